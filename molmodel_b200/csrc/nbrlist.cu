@@ -115,7 +115,9 @@ __global__ void __launch_bounds__(kCheckThreads) k_list_check(const double *__re
     } else if (d > b) {
       b = d;
     }
-    if (prune > 0) {
+    // before the first build there are no ranks to read (and the rows are made
+    // anew whatever the moves)
+    if (prune > 0 && !first) {
       const int p = rank[g];
       const double ex = x - plast[3 * p], ey = y - plast[3 * p + 1], ez = z - plast[3 * p + 2];
       const double e = ex * ex + ey * ey + ez * ez;
