@@ -485,8 +485,7 @@ extern "C" int mmnb_site_gradients(mmnb_handle *h, const double *dl_df, double *
                      "no evaluation to differentiate: call mmnb_forward first (any other evaluation, "
                      "mmnb_set_params or mmnb_scale since then discards it)");
   const size_t n = h->nsite, n3 = 3 * n;
-  const size_t nskd = h->kspace ? 2 * (size_t) h->nk : 0;
-  const size_t need = kGradSlots * n + n3 + nskd;
+  const size_t need = kGradSlots * n + n3;
   if (h->bwd_cap < need) {
     if (h->d_bwd)
       cudaFree(h->d_bwd);
@@ -503,7 +502,6 @@ extern "C" int mmnb_site_gradients(mmnb_handle *h, const double *dl_df, double *
     h->bwd_cap = need;
   }
   double *d_out = h->d_bwd, *d_g = dl_df ? h->d_bwd + kGradSlots * n : nullptr;
-  double *d_skd = h->d_bwd + kGradSlots * n + n3;
   P3mScratch ps;
   const bool p3m = h->any_q && h->cfg.include_kspace && h->p3m && dl_df;
   if (p3m) {
@@ -575,7 +573,7 @@ extern "C" int mmnb_site_gradients(mmnb_handle *h, const double *dl_df, double *
     if (h->p3m)
       e = launch_p3m_dipole_fp64(h, h->d_r, d_g, ps, d_out + kDlDq * n);
     else if (h->kspace)
-      e = launch_kspace_dipole(h, h->d_r, d_g, d_skd, d_out + kDlDq * n);
+      e = launch_kspace_dipole(h, h->d_r, d_g, d_out + kDlDq * n);
   }
   if (e == cudaSuccess) {
     k_grad_finish<<<div_up(h->nsite, kGradThreads), kGradThreads, 0, h->stream>>>(h->nsite, h->d_mask, h->d_eps,

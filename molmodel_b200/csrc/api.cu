@@ -330,44 +330,14 @@ int setup_cheb(mmnb_handle *h)
   return upload(h, &h->d_cheb_d, d4);
 }
 
-// reciprocal lattice 2 pi inv(latv)^T of the diagonal box
-void recip_diag(const mmnb_handle *h, double rec[3])
-{
-  for (int d = 0; d < 3; d++)
-    rec[d] = 2 * M_PI * (1.0 / h->box.L[d]);
-}
-
 // ordinary Ewald wave vectors (src/kspace.c:35-71, 96-103)
 int setup_kspace(mmnb_handle *h)
 {
-  const double kc = h->cfg.kspace_cutoff;
-  const double n2max = kc * kc + 1e-8;
-  const int nmax = (int) floor(kc);
-  struct KI { int x, y, z, n2; };
-  std::vector<KI> ks;
-  for (int nx = 0; nx <= nmax; nx++)
-    for (int ny = (nx == 0 ? 0 : -nmax); ny <= nmax; ny++)
-      for (int nz = (nx == 0 && ny == 0 ? 1 : -nmax); nz <= nmax; nz++)
-        if (nx * nx + ny * ny + nz * nz <= n2max)
-          ks.push_back(KI{nx, ny, nz, nx * nx + ny * ny + nz * nz});
-  std::stable_sort(ks.begin(), ks.end(), [](const KI &a, const KI &b) { return a.n2 > b.n2; });
-  h->nk = (int) ks.size();
-  h->kmax = nmax;
-  double rec[3];
-  recip_diag(h, rec);
-  std::vector<double> kv(3 * ks.size()), ak(ks.size());
-  const double c = 0.25 / (h->eta * h->eta), f = 4 * M_PI / h->volume;
-  for (size_t k = 0; k < ks.size(); k++) {
-    kv[3 * k] = rec[0] * ks[k].x;
-    kv[3 * k + 1] = rec[1] * ks[k].y;
-    kv[3 * k + 2] = rec[2] * ks[k].z;
-    const double k2 = kv[3 * k] * kv[3 * k] + kv[3 * k + 1] * kv[3 * k + 1] + kv[3 * k + 2] * kv[3 * k + 2];
-    ak[k] = f * exp(-k2 * c) / k2;
-  }
-  int s;
-  if ((s = upload(h, &h->d_kvecs, kv)) || (s = upload(h, &h->d_ak, ak)) ||
-      (s = dalloc(h, &h->d_skc, 2 * ks.size())))
-    return s;
+  h->buf_gen++;
+  const cudaError_t e = ewald_make(h, h->ew);
+  if (e == cudaErrorInvalidValue)
+    return fail(h, MMNB_ERR_ARG, "kspace_cutoff is too large");
+  CK(e);
   return MMNB_OK;
 }
 
@@ -533,12 +503,13 @@ void free_all(mmnb_handle *h)
                   h->d_sp, h->d_site_of_slot,
                   h->d_phi, h->d_evec, h->d_ljf, h->d_lj_part, h->d_elec_part, h->d_energy, h->d_r, h->d_f,
                   h->d_mesh, h->d_meshk, h->d_green, h->d_kvec, h->d_egrid, h->d_egridk, h->d_mesh32,
-                  h->d_meshk32, h->d_green32, h->d_egrid32, h->d_egridk32, h->d_mesh_fx, h->d_kint, h->d_kvecs, h->d_ak, h->d_skc,
+                  h->d_meshk32, h->d_green32, h->d_egrid32, h->d_egridk32, h->d_mesh_fx,
                   h->mx.site, h->mx.par, h->mx.anchor, h->mx.anc32, h->mx.acc, h->mx.acck, h->d_wsum,
-                  h->d_bwd, h->d_gmesh, h->d_gmeshk, h->d_chi_part};
+                  h->d_bwd, h->d_esp, h->d_gmesh, h->d_gmeshk, h->d_chi_part};
   for (void *p : ptrs)
     if (p)
       cudaFree(p);
+  ewald_free(h->ew);
   if (h->side) {
     cudaStreamSynchronize(h->side);
     cudaStreamDestroy(h->side);
@@ -1066,6 +1037,23 @@ int mmnb_compute_device(mmnb_handle *h, const double *d_r, double *d_f, double *
     if (h->timing.on)
       CK(cudaStreamWaitEvent(main, h->ev_join, 0));
   }
+  // the k-sum's structure factor depends only on the positions too; its field
+  // joins the site arrays after the pair kernels
+  const bool ksum = h->any_q && h->cfg.include_kspace && h->kspace && h->ew.nk > 0;
+  if (ksum && h->tune.p3m_side) {
+    cudaStream_t main = h->stream;
+    CK(cudaEventRecord(h->ev_fork, main));
+    CK(cudaStreamWaitEvent(h->side, h->ev_fork, 0));
+    if (h->in_chunks)
+      CK(cudaStreamWaitEvent(h->side, h->ev_in[mmnb_handle::kInChunks - 1], cudaEventWaitExternal));
+    h->stream = h->side;
+    const cudaError_t e = launch_ewald_structure(h, h->ew, d_r, nullptr);
+    h->stream = main;
+    CK(e);
+    CK(cudaEventRecord(h->ev_join, h->side));
+    if (h->timing.on)
+      CK(cudaStreamWaitEvent(main, h->ev_join, 0));
+  }
   if (h->in_chunks)
     CK(cudaStreamWaitEvent(h->stream, h->ev_in[mmnb_handle::kInChunks - 1], cudaEventWaitExternal));
   if (p3m && !side)
@@ -1117,8 +1105,12 @@ int mmnb_compute_device(mmnb_handle *h, const double *d_r, double *d_f, double *
     if (!mixed)
       CK(launch_p3m_fp64(h, d_r, 2));
     timing_mark(h, "kspace");
-  } else if (h->any_q && h->cfg.include_kspace && h->kspace) {
-    CK(launch_kspace(h, d_r));
+  } else if (ksum) {
+    if (!h->tune.p3m_side)
+      CK(launch_ewald_structure(h, h->ew, d_r, nullptr));
+    else if (!h->timing.on)
+      CK(cudaStreamWaitEvent(h->stream, h->ev_join, 0));
+    CK(launch_ewald_sum(h, h->ew, h->nsite, d_r, 0.0, h->d_phi, h->d_evec));
     timing_mark(h, "kspace");
   }
   CK(launch_finalize(h, d_f, energy));
@@ -1419,6 +1411,7 @@ int mmnb_scale(mmnb_handle *h, double s)
     if (h->cfg.precision == MMNB_MIXED)
       CK(launch_green32(h));
   }
+  ewald_free(h->ew);
   if (h->kspace && (st = setup_kspace(h)))
     return st;
   if ((st = setup_cells(h)))

@@ -73,6 +73,18 @@ struct MixedBufs {
   long long *acck = nullptr;     // per site (original order): P3M interpolation phi, Ex, Ey, Ez
 };
 
+// Wave vectors and sums of the ordinary Ewald reciprocal space (kspace.cu)
+struct EwaldSum {
+  bool made = false;
+  int nk = 0, nrow = 0, nmax = 0;
+  double rec[3] = {0, 0, 0};
+  int4 *row = nullptr;      // rows of consecutive n_z: (n_x, n_y, first n_z, its index)
+  short4 *kint = nullptr;   // integer n of each wave vector
+  double *ak2 = nullptr;    // 2 a_k
+  double2 *sk = nullptr;    // 2 a_k S(k)
+  double2 *part = nullptr;  // partial S(k) of the structure factor's blocks
+};
+
 // Stage timing with CUDA events recorded on the handle's stream.  Each
 // evaluation starts with a "start" mark; a stage's time is the interval from
 // the previous mark to its own.
@@ -204,11 +216,13 @@ struct mmnb_handle {
   // [3]: row counter of the FP64 water kernel; [4]: the mixed water kernel's
   // fixed-point virial term
   unsigned long long *d_wsum = nullptr;
-  // parameter gradients (allocated on first use): six per-site outputs, dL/dF,
-  // the dipole structure factor of the reciprocal sum
+  // parameter gradients (allocated on first use): six per-site outputs, dL/dF
   double *d_bwd = nullptr;
   size_t bwd_cap = 0;
   double *h_bwd = nullptr;  // pinned: the gradient slots come back in one copy
+  // potential at points: scratch kept from call to call (at most 64 MB)
+  double *d_esp = nullptr;
+  size_t esp_cap = 0;
   bool grad_ready = false;           // the last evaluation was mmnb_forward's and nothing changed since
   // FP64 dipole solve for a mixed-form handle, which has no FP64 meshes or plans
   double *d_gmesh = nullptr;
@@ -253,11 +267,7 @@ struct mmnb_handle {
 
   // ordinary Ewald
   bool kspace = false;
-  int nk = 0, kmax = 0;
-  int *d_kint = nullptr;             // 3 per k
-  double *d_kvecs = nullptr;         // 3 per k
-  double *d_ak = nullptr;
-  double *d_skc = nullptr;           // 2 per k: sum q cos, sum q sin
+  mmnb::EwaldSum ew;                 // made with the handle, or on the first potential at points
 
   // mixed form
   mmnb::MixedBufs mx;
@@ -330,9 +340,8 @@ struct P3mScratch {
 // d_psi += mesh potential of the dipoles q_j g_j (g: 3 per site), FP64
 cudaError_t launch_p3m_dipole_fp64(mmnb_handle *h, const double *d_r, const double *d_g, const P3mScratch &s,
                                    double *d_psi);
-// d_psi += reciprocal-sum potential of the dipoles q_j g_j; d_skd: 2 per k
-cudaError_t launch_kspace_dipole(mmnb_handle *h, const double *d_r, const double *d_g, double *d_skd,
-                                 double *d_psi);
+// d_psi += reciprocal-sum potential of the dipoles q_j g_j
+cudaError_t launch_kspace_dipole(mmnb_handle *h, const double *d_r, const double *d_g, double *d_psi);
 cudaError_t launch_p3m_mixed(mmnb_handle *h, const double *d_r, int stage);
 // write back and drop [p, p + bytes) from the host cores' caches (hostmem.cpp)
 void evict_host_lines(const void *p, size_t bytes);
@@ -342,7 +351,14 @@ void evict_host_lines(const void *p, size_t bytes);
 // pieces give the mesh of one launch over all sites, bit for bit)
 cudaError_t launch_spread_mixed_range(mmnb_handle *h, const double *d_r, int lo, int hi);
 cudaError_t launch_green32(mmnb_handle *h);
-cudaError_t launch_kspace(mmnb_handle *h, const double *d_r);
+// wave vectors of the handle's kspace_cutoff, eta and box (drops what e held)
+cudaError_t ewald_make(mmnb_handle *h, EwaldSum &e);
+void ewald_free(EwaldSum &e);
+// S(k) of the sites at d_r (with d_g: of the dipoles q g) into e.sk
+cudaError_t launch_ewald_structure(mmnb_handle *h, const EwaldSum &e, const double *d_r, const double *d_g);
+// d_phi += potential of e.sk at the n points, + neutral; d_evec (or null) += the field
+cudaError_t launch_ewald_sum(mmnb_handle *h, const EwaldSum &e, int n, const double *d_pts, double neutral,
+                             double *d_phi, double *d_evec);
 cudaError_t launch_finalize(mmnb_handle *h, double *d_f, double *d_energy);
 cudaError_t launch_energy(mmnb_handle *h, double *d_energy);
 
