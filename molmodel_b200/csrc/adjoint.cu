@@ -46,11 +46,10 @@ constexpr int kGradQueue = 64;  // per warp: at most 31 carried over plus 32 new
 enum GradSlot { kDuDq = 0, kDuDsig, kDuDeps, kDlDq, kDlDsig, kDlDeps, kGradSlots };
 
 struct GradArgs {
-  int nsite, ngroup, rowcap, geometric;
+  int nsite, ngroup, rowcap, geometric, series;
   Box box;
   double rlo2, rhi2, inv_sw, eta;
   double cheb_min, cheb_max, cheb_inv_dx;
-  const double *cheb;
   // the rigid-water forward's copy of the table: the cubics' (c0, c1) and
   // (c2, c3), continued to (rc + 2.5)^2 (k_grad_pair)
   const double2 *tw0, *tw1;
@@ -106,6 +105,8 @@ __device__ __forceinline__ void ewald_grad_b(const GradArgs &a, double r2, doubl
     const double2 c01 = __ldg(a.tw0 + i), c23 = __ldg(a.tw1 + i);
     b0 = ((c23.y * f + c23.x) * f + c01.y) * f + c01.x;
     b1 = -2 * a.cheb_inv_dx * ((3 * c23.y * f + 2 * c23.x) * f + c01.y);
+  } else if (x <= 0 && a.series) {
+    ewald_short(a.eta * a.eta, a.eta * M_2_SQRTPI, r2, b0, b1);
   } else {
     const double r = sqrt(r2);
     const double er = a.eta * r;
@@ -522,7 +523,7 @@ extern "C" int mmnb_site_gradients(mmnb_handle *h, const double *dl_df, double *
   a.cheb_min = h->cheb_min;
   a.cheb_max = h->cheb_max;
   a.cheb_inv_dx = h->cheb_inv_dx;
-  a.cheb = h->d_cheb;
+  a.series = h->eta * sqrt(h->cheb_min) <= kErfSeriesMax;
   a.tw0 = reinterpret_cast<const double2 *>(h->d_cheb_w);
   a.tw1 = a.tw0 + h->cheb_w_nseg;
   a.nsegw = h->cheb_w_nseg;

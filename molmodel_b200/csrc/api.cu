@@ -287,14 +287,9 @@ int initial_rowcap(const mmnb_handle *h)
 
 int setup_cheb(mmnb_handle *h)
 {
-  std::vector<double> c7(kCheb * 7), c8(kCheb * 8, 0.0);
+  std::vector<double> c7(kCheb * 7);
   chebyshev_table(h->rc, h->eta, &h->cheb_min, &h->cheb_max, &h->cheb_inv_dx, c7.data());
-  for (int i = 0; i < kCheb; i++)
-    for (int k = 0; k < 7; k++)
-      c8[8 * i + k] = c7[7 * i + k];
-  int s = upload(h, &h->d_cheb, c8);
-  if (s)
-    return s;
+  int s;
   // the rigid-water FP64 kernel's copy: the cubic's coefficients only, as two
   // arrays of (c0, c1) and (c2, c3), continued to (rc + 2.5)^2 so every site
   // pair of a water group pair within rc falls inside it
@@ -313,7 +308,6 @@ int setup_cheb(mmnb_handle *h)
     w[2 * ((size_t) h->cheb_w_nseg + i)] = o[2];
     w[2 * ((size_t) h->cheb_w_nseg + i) + 1] = o[3];
   }
-  h->water64_grid = 0;  // the kernel's shared-memory size follows the table
   if ((s = upload(h, &h->d_cheb_w, w)))
     return s;
   // the same fit of (2 eta / sqrt(pi)) exp(-eta^2 r^2) = -eta d/d(eta) of
@@ -495,12 +489,12 @@ void free_all(mmnb_handle *h)
     h->copy_in = nullptr;
   }
   void *ptrs[] = {h->d_group, h->d_excl_ptr, h->d_excl_idx, h->d_p14_ptr, h->d_p14_idx, h->d_gexcl_ptr,
-                  h->d_gexcl_idx, h->d_mask, h->d_q, h->d_sig, h->d_eps, h->d_rscreen, h->d_cheb, h->d_cheb_w, h->d_cheb_d, h->d_lj_row, h->d_lj_row_part,
+                  h->d_gexcl_idx, h->d_mask, h->d_q, h->d_sig, h->d_eps, h->d_rscreen, h->d_cheb_w, h->d_cheb_d, h->d_lj_row, h->d_lj_row_part,
                   h->d_vir_part, h->d_vir_row, h->d_vir_mol, h->d_vir_molw, h->d_vir_mass,
                   h->d_stencil, h->d_cell_rank, h->d_cell_of_rank, h->d_cell_of_group, h->d_cell_count,
                   h->d_cell_start, h->d_slot, h->d_sorted, h->d_rank, h->d_anchor, h->d_last, h->d_anchor_sorted, h->d_anchor32, h->d_block_sum,
                   h->d_top2, h->d_nbr, h->d_nbr_count, h->d_pnbr, h->d_pcount, h->d_plast, h->d_flags, h->d_sr,
-                  h->d_sp, h->d_site_of_slot,
+                  h->d_sp, h->d_sanchor, h->d_site_of_slot,
                   h->d_phi, h->d_evec, h->d_ljf, h->d_lj_part, h->d_elec_part, h->d_energy, h->d_r, h->d_f,
                   h->d_mesh, h->d_meshk, h->d_green, h->d_kvec, h->d_egrid, h->d_egridk, h->d_mesh32,
                   h->d_meshk32, h->d_green32, h->d_egrid32, h->d_egridk32, h->d_mesh_fx,
@@ -785,6 +779,7 @@ static int create_impl(mmnb_handle *h, const mmnb_config *c, int nsite, int ngro
     return s;
   const size_t nslot = (size_t) ngroup * h->G;
   if ((s = dalloc(h, &h->d_sr, nslot)) || (s = dalloc(h, &h->d_sp, nslot)) ||
+      (s = dalloc(h, &h->d_sanchor, ngroup)) ||
       (s = dalloc(h, &h->d_site_of_slot, nslot)))
     return s;
   h->elec_blocks = div_up(nsite, 256);
@@ -959,6 +954,8 @@ int mmnb_set_params(mmnb_handle *h, const int *site_mask, const double *q, const
     h->uni_qH = (float) q[a + 1];
     h->uni_sig = (float) sig[a];
     h->uni_seps = (float) sqrt(eps[a]);
+    const double u[4] = {q[a], q[a + 1], sig[a], sqrt(eps[a])};
+    std::copy(u, u + 4, h->uni64);
   }
   h->params_set = true;
   return MMNB_OK;
@@ -1076,7 +1073,7 @@ int mmnb_compute_device(mmnb_handle *h, const double *d_r, double *d_f, double *
     CK(launch_sort_sites(h, d_r));
   timing_mark(h, "sort_sites");
   h->used_water = false;
-  h->used_water64 = false;
+  h->used_rows64 = false;
   if (h->cfg.include_rspace) {
     if (mixed && h->water && !h->want_fields) {
       CK(launch_rspace_water(h));
@@ -1085,9 +1082,10 @@ int mmnb_compute_device(mmnb_handle *h, const double *d_r, double *d_f, double *
       CK(launch_rspace_mixed(h));
     } else if (water64) {
       CK(launch_rspace_water64(h));
-      h->used_water64 = true;
+      h->used_rows64 = true;
     } else {
       CK(launch_rspace_fp64(h));
+      h->used_rows64 = true;
     }
     timing_mark(h, "rspace_pair");
     if (!excl_side) {

@@ -121,10 +121,11 @@ struct mmnb_handle {
   // same charge (the rigid-water kernel then copies only the H offsets)
   bool water_uni = false;
   float uni_qO = 0, uni_qH = 0, uni_sig = 0, uni_seps = 0;
+  double uni64[4] = {0, 0, 0, 0};    // the same in FP64
   bool want_fields = false;          // this evaluation must produce per-site potential and field
   bool want_virial = false;          // this evaluation's pair kernels also sum the virial's pair term
   bool used_water = false;           // the last evaluation ran the water kernel
-  bool used_water64 = false;         // the last evaluation ran the FP64 water kernel
+  bool used_rows64 = false;          // the last evaluation ran an FP64 pair kernel: energies per row
   double totA = 0, totB = 0, lj_correction = 0, neutral_b = 0;
 
   // host topology
@@ -141,16 +142,12 @@ struct mmnb_handle {
   int *d_gexcl_ptr = nullptr, *d_gexcl_idx = nullptr;
   int *d_mask = nullptr;
   double *d_q = nullptr, *d_sig = nullptr, *d_eps = nullptr, *d_rscreen = nullptr;
-  double *d_cheb = nullptr;          // 512 x 8 doubles (7 used) + nothing else
   double cheb_min = 0, cheb_max = 0, cheb_inv_dx = 0;
   // the rigid-water FP64 kernel's table: cheb_w_nseg x (c0, c1), then x (c2, c3)
   double *d_cheb_w = nullptr;
   int cheb_w_nseg = 0;
   // 512 x 4: the cubics of -eta d/d(eta) of the table (mmnb_virial)
   double *d_cheb_d = nullptr;
-  int water64_grid = 0;              // persistent blocks of that kernel (0: not sized yet)
-  int water64_warps = 0;             // warps per block of that kernel
-  size_t water64_smem = 0;
 
   // neighbour list
   mmnb::CellGeom cg{};
@@ -195,8 +192,9 @@ struct mmnb_handle {
   int force_rebuild_next = 0;
 
   // sorted, padded site data (FP64 form)
-  double4 *d_sr = nullptr;           // ngroup*G sites: x, y, z, q
-  double4 *d_sp = nullptr;           // sig, eps, rscreen, (mask as double)
+  double4 *d_sr = nullptr;           // ngroup*G sites: offset from the anchor, q
+  double4 *d_sp = nullptr;           // sig, sqrt(eps), rscreen, -
+  double4 *d_sanchor = nullptr;      // sorted groups: anchor, first site and site masks
   int *d_site_of_slot = nullptr;     // ngroup*G -> original site (or -1)
 
   // outputs (original order)
@@ -386,61 +384,30 @@ __device__ __forceinline__ bool csr_has(const int *ptr, const int *idx, int row,
   return false;
 }
 
-// b0 = erfc(eta r)/r, b1 = (b0 + 2 eta/sqrt(pi) exp(-eta^2 r^2)) / r^2 from the
-// reference's 512-segment Chebyshev table (8 doubles per segment) inside
-// (cmin, cmax), from erfc/exp outside it; seg and f: the table segment and the
-// position in it (seg = -1 outside the table)
-__device__ __forceinline__ void ewald_table_b(const double *cheb, double cmin, double cmax, double inv_dx,
-                                              double eta, double r2, double &b0, double &b1, int &seg, double &f)
-{
-  if (cmin < r2 && r2 < cmax) {
-    double x = (r2 - cmin) * inv_dx;
-    const unsigned i = (unsigned) x;
-    const double2 *c = reinterpret_cast<const double2 *>(cheb + 8 * (size_t) i);
-    const double2 c01 = __ldg(c), c23 = __ldg(c + 1), c45 = __ldg(c + 2), c67 = __ldg(c + 3);
-    x -= i;
-    b0 = ((c23.y * x + c23.x) * x + c01.y) * x + c01.x;
-    b1 = (c67.x * x + c45.y) * x + c45.x;
-    seg = (int) i;
-    f = x;
-  } else {
-    const double r = sqrt(r2);
-    const double er = eta * r;
-    const double e = exp(-(er * er));
-    b0 = erfc(er) / r;
-    b1 = (b0 + eta * M_2_SQRTPI * e) / r2;
-    seg = -1;
-    f = 0;
-  }
-}
+// (-1)^n / (n! (2n + 1)): erf(x) = 2 x / sqrt(pi) sum_n of these x^(2n)
+static __constant__ double kErfSeries[16] = {
+    1.0, -1.0 / 3, 1.0 / 10, -1.0 / 42, 1.0 / 216, -1.0 / 1320, 1.0 / 9360, -1.0 / 75600, 1.0 / 685440,
+    -1.0 / 6894720, 1.0 / 76204800, -1.0 / 918086400, 1.0 / 11975040000.0, -1.0 / 168129561600.0,
+    1.0 / 2528170444800.0, -1.0 / 40537905408000.0};
 
-// The same from the cubic alone: t0[i] = (c0, c1), t1[i] = (c2, c3) of segment i
-// (the rigid-water kernels' copy of the table, whose first 512 segments are the
-// reference's), b1 from the cubic's derivative -- the reference stores b1's
-// quadratic as exactly -2 k c_k / dx (k = 1..3), so the two differ only in
-// rounding.  Same range, segment and position as ewald_table_b; half the reads.
-__device__ __forceinline__ void ewald_table_half(const double2 *t0, const double2 *t1, double cmin, double cmax,
-                                                 double inv_dx, double eta, double r2, double &b0, double &b1,
-                                                 int &seg, double &f)
+// b0 = erfc(eta r)/r and b1 = -2 d b0 / d(r^2) for r^2 below the table, where
+// eta r <= kErfSeriesMax: b0 = 1/r - erf(eta r)/r, from erf's Maclaurin series
+// (16 terms: the first one left out is below 1e-17 of the sum).  A few site pairs
+// of a row take this branch and the rest of the warp waits for them: 45 FP64
+// operations here, several hundred for erfc and exp (rigid-water FP64 kernel 259 ->
+// 226 us on 32,768 waters).
+constexpr double kErfSeriesMax = 0.85;
+__device__ __forceinline__ void ewald_short(double eta2, double two_eta_rsqrtpi, double r2, double &b0, double &b1)
 {
-  if (cmin < r2 && r2 < cmax) {
-    double x = (r2 - cmin) * inv_dx;
-    const unsigned i = (unsigned) x;
-    const double2 c01 = __ldg(t0 + i), c23 = __ldg(t1 + i);
-    x -= i;
-    b0 = ((c23.y * x + c23.x) * x + c01.y) * x + c01.x;
-    b1 = -2 * inv_dx * ((3 * c23.y * x + 2 * c23.x) * x + c01.y);
-    seg = (int) i;
-    f = x;
-  } else {
-    const double r = sqrt(r2);
-    const double er = eta * r;
-    const double e = exp(-(er * er));
-    b0 = erfc(er) / r;
-    b1 = (b0 + eta * M_2_SQRTPI * e) / r2;
-    seg = -1;
-    f = 0;
+  const double y = eta2 * r2, rinv = rsqrt(r2);
+  double p = kErfSeries[15], d = 0;
+#pragma unroll
+  for (int n = 14; n >= 0; n--) {
+    d = fma(d, y, p);
+    p = fma(p, y, kErfSeries[n]);
   }
+  b0 = fma(-two_eta_rsqrtpi, p, rinv);
+  b1 = fma(2 * two_eta_rsqrtpi * eta2, d, rinv * rinv * rinv);
 }
 
 // minimum image of one site displacement, rounded as the reference rounds it
@@ -468,6 +435,16 @@ __device__ __forceinline__ double anchor_disp(const Box &b, double4 ri, double4 
 }
 
 #endif
+
+// Segments of the continued table the FP64 pair kernels use.  Past 1.2 rc^2 the
+// reference evaluates erfc and exp; the cubics continued there are within ~1e-9 of
+// those, relatively, which is below 1e-12 of the pair's terms once erfc(eta r) has
+// fallen below ~4e-4 (eta rc >= 2.3, as any screening that makes the cutoff worth
+// anything has it).  Below that the kernels, too, take the exact functions.
+inline double table_segments(const mmnb_handle *h)
+{
+  return h->eta * h->rc >= 2.3 ? h->cheb_w_nseg : kCheb;
+}
 
 inline int div_up(long a, long b) { return (int) ((a + b - 1) / b); }
 

@@ -19,47 +19,53 @@
 //     erfc, is what reproduces the reference);
 //   * past the table's upper end (r^2 > 1.2 rc^2, which only site pairs of
 //     water reach) the table continues with segments of the same construction
-//     (the reference evaluates erfc and exp there; the two differ by ~1e-16
-//     absolute at those distances), and below its lower end (r^2 < 4) erfc and
-//     exp are evaluated directly, as in the reference.
+//     where that is as good as the erfc and exp the reference evaluates there
+//     (table_segments), and below its lower end (r^2 < 4) they are exact
+//     (ewald_short).
 //
-// Layout: a persistent grid, one block of up to kW64Warps warps per SM slot; each
+// Layout: a persistent grid, one block of up to kW64Warps warps per SM; each
 // warp takes the next row group from a counter and walks its list 32 entries
 // at a time (anchor test per lane, ballot compaction into a 128-slot ring of
-// anchor displacements, cp.async of the partner's 96-byte record into the same
-// slot), evaluating 32 queued group pairs at a time.  The table's two halves,
+// anchor displacements, cp.async of the partner's record -- its H offsets where
+// every water has the same parameters -- into the same slot, an array per 16-byte
+// word), evaluating 32 queued group pairs at a time.  The table's two halves,
 // (c0, c1) and (c2, c3) per segment, sit in shared memory as two arrays of
-// 16-byte entries, so a warp's random segment reads spread over all banks.
-// Row totals are summed over the lanes in a fixed order (transpose through
-// shared memory), so results do not depend on which warp or SM took the row.
+// 16-byte entries in up to eight interleaved copies (a lane reads copy lane mod
+// copies, so that the eight lanes of an access phase meet in a bank less often;
+// four fit beside twelve warps' rings at rc 9).  Row totals are summed over the
+// lanes in a fixed order (transpose through shared memory), so results do not
+// depend on which warp or SM took the row.
+//
+// Bound by the shared-memory pipe and FP64 latency at 12 warps per SM.  On 32,768
+// waters: 259 us with 32-byte ring words, one table and erfc below it; 226 with
+// erf's series there (ewald_short); 191 with word arrays, records of H offsets and
+// four copies.  On one row per warp the table's copy-in shows: asynchronous, 21 -> 17
+// us on 216 waters.
 
 #include "mmnb_internal.cuh"
 
+#include <algorithm>
+
 namespace mmnb {
 
-#ifndef MMNB_W64_BLOCKS
-#define MMNB_W64_BLOCKS 1
-#endif
 // warps per block the kernel is compiled for (its register budget: 12 warps
 // of 384 threads leave 170 registers a thread); a launch may use fewer when
 // the rings and the table do not fit in shared memory
-#ifndef MMNB_W64_WARPS
-#define MMNB_W64_WARPS 12
-#endif
-constexpr int kW64Warps = MMNB_W64_WARPS;
+constexpr int kW64Warps = 12;
 // a batch of 32 is queued before the oldest 32 are evaluated, so the ring
 // holds up to 63 + 32 entries
 constexpr int kW64Ring = 128;
 constexpr int kW64Acc = 17;  // phi (3), field (9), LJ + switch force on O (3), LJ energy, virial term
 
 struct Water64Args {
-  int ngroup, rowcap, geometric, nseg;
+  int ngroup, rowcap, geometric, nseg, copies, series;
   Box box;
   double rlo2, rhi2, inv_sw, eta;
   double cmin, inv_dx, dscale, nsegd;  // dscale = -2 / segment width
   const double2 *table;                // [nseg] (c0, c1), then [nseg] (c2, c3)
   const double4 *anchor;               // sorted groups: anchor (x, y, z, -)
-  const double4 *rec;                  // sorted groups: 3 x double4, layout in k_sort_water64
+  const double2 *rec;                  // sorted groups: 6 x double2, layout in k_sort_water64
+  double qO, qH, sig, seps;            // uniform water: charges and LJ parameters
   const int *nbr, *nbr_count, *sorted, *group;
   unsigned long long *counter;         // next row; zeroed by k_sort_water64
   double *phi, *evec, *ljf, *lj_row;
@@ -79,16 +85,20 @@ __device__ __forceinline__ void ewald_w64(const Water64Args &a, const double2 *t
     const int i = __double2loint(t);
     f = x - (t - 4503599627370496.0);
     seg = i;
-    const double2 c01 = t0[i], c23 = t1[i];
+    const double2 c01 = t0[i * a.copies], c23 = t1[i * a.copies];
     b0 = ((c23.y * f + c23.x) * f + c01.y) * f + c01.x;
     b1 = a.dscale * ((3 * c23.y * f + 2 * c23.x) * f + c01.y);
   } else {
     seg = -1;
     f = 0;
-    const double r = sqrt(r2);
-    const double er = a.eta * r;
-    b0 = erfc(er) / r;
-    b1 = (b0 + a.eta * M_2_SQRTPI * exp(-(er * er))) / r2;
+    if (x <= 0 && a.series) {
+      ewald_short(a.eta * a.eta, a.eta * M_2_SQRTPI, r2, b0, b1);
+    } else {
+      const double r = sqrt(r2);
+      const double er = a.eta * r;
+      b0 = erfc(er) / r;
+      b1 = (b0 + a.eta * M_2_SQRTPI * exp(-(er * er))) / r2;
+    }
   }
 }
 
@@ -127,19 +137,41 @@ __device__ __forceinline__ void cp16(void *dst, const void *src)
                : "memory");
 }
 
-template <bool VIR>
-__global__ void __launch_bounds__(kW64Warps * 32, MMNB_W64_BLOCKS) k_pair_water64(Water64Args a)
+// 16-byte words of a queued partner: anchor displacement and r^2, H offsets and,
+// unless every water has the same parameters, charges and LJ parameters
+constexpr int w64_words(bool uni) { return uni ? 5 : 8; }
+
+// UNI: every water has the same parameters (taken from the arguments)
+template <bool VIR, bool UNI>
+__global__ void __launch_bounds__(kW64Warps * 32, 1) k_pair_water64(Water64Args a)
 {
+  constexpr int kWords = w64_words(UNI);
   extern __shared__ __align__(16) unsigned char smem[];
-  // per warp: ring of (anchor displacement, r^2) and the partner's record
-  double4 *ring = reinterpret_cast<double4 *>(smem);  // [warps][4][kW64Ring]
-  double2 *tc01 = reinterpret_cast<double2 *>(smem + sizeof(double4) * 4 * kW64Ring * (blockDim.x >> 5));
-  const double2 *tc23 = tc01 + a.nseg;
-  for (int i = threadIdx.x; i < 2 * a.nseg; i += blockDim.x)
-    tc01[i] = a.table[i];
-  __syncthreads();
+  // per warp: ring of (x, y), (z, r^2) of the anchor displacement and the partner's
+  // record, one array per 16-byte word: consecutive lanes read consecutive words
+  double2 *ring = reinterpret_cast<double2 *>(smem);  // [warps][kWords][kW64Ring]
+  double2 *tab = ring + (size_t) kWords * kW64Ring * (blockDim.x >> 5);
+  // the table is on its way while the first rows are walked: each warp waits for it
+  // (and meets the block) before its first evaluation
+  bool table_ready = false;
+  if (a.copies == 1) {
+    for (int i = threadIdx.x; i < 2 * a.nseg; i += blockDim.x)
+      cp16(tab + i, a.table + i);
+  } else {
+    for (int i = threadIdx.x; i < 2 * a.nseg * a.copies; i += blockDim.x)
+      tab[i] = a.table[i / a.copies];
+  }
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  auto wait_table = [&]() {
+    if (table_ready)
+      return;
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    table_ready = true;
+  };
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  double4 *qa = ring + (size_t) w * 4 * kW64Ring, *q0 = qa + kW64Ring, *q1 = q0 + kW64Ring, *q2 = q1 + kW64Ring;
+  const double2 *const tc01 = tab + lane % a.copies, *const tc23 = tc01 + a.nseg * a.copies;
+  double2 *const q = ring + (size_t) w * kWords * kW64Ring;
   const unsigned below = (1u << lane) - 1;
   for (;;) {
     int p = 0;
@@ -149,18 +181,34 @@ __global__ void __launch_bounds__(kW64Warps * 32, MMNB_W64_BLOCKS) k_pair_water6
     if (p >= a.ngroup)
       break;
     const double4 ai = a.anchor[p];
-    const double4 r0 = a.rec[3 * (size_t) p], r1 = a.rec[3 * (size_t) p + 1], r2 = a.rec[3 * (size_t) p + 2];
-    // record: (h1x, h1y, h1z, h2x), (h2y, h2z, qO, qH1), (qH2, sigma, sqrt(eps), -)
-    const double h1x = r0.x, h1y = r0.y, h1z = r0.z, h2x = r0.w, h2y = r1.x, h2z = r1.y;
-    const double qO = r1.z, qH1 = r1.w, qH2 = r2.x, sgO = r2.y, seO = r2.z;
+    // record: (h1x, h1y), (h1z, h2x), (h2y, h2z), (qO, qH1), (qH2, sigma), (sqrt(eps), -)
+    const double2 *const rp = a.rec + 6 * (size_t) p;
+    const double2 r0 = rp[0], r1 = rp[1], r2 = rp[2];
+    double2 r3 = make_double2(a.qO, a.qH), r4 = make_double2(a.qH, a.sig), r5 = make_double2(a.seps, 0.0);
+    if (!UNI) {
+      r3 = rp[3];
+      r4 = rp[4];
+      r5 = rp[5];
+    }
+    const double h1x = r0.x, h1y = r0.y, h1z = r1.x, h2x = r1.y, h2y = r2.x, h2z = r2.y;
+    const double qO = r3.x, qH1 = r3.y, qH2 = r4.x, sgO = r4.y, seO = r5.x;
     double acc[kW64Acc];
 #pragma unroll
     for (int c = 0; c < kW64Acc; c++)
       acc[c] = 0;
     auto compute = [&](int k) {
-      const double4 da = qa[k], j0 = q0[k], j1 = q1[k], j2 = q2[k];
-      const double j1x = j0.x, j1y = j0.y, j1z = j0.z, j2x = j0.w, j2y = j1.x, j2z = j1.y;
-      const double qjO = j1.z, qj1 = j1.w, qj2 = j2.x, sgj = j2.y, sej = j2.z;
+      const double2 *const e = q + k;
+      const double2 d0 = e[0], d1 = e[kW64Ring], j0 = e[2 * kW64Ring], j1 = e[3 * kW64Ring], j2 = e[4 * kW64Ring];
+      double2 j3 = make_double2(a.qO, a.qH), j4 = make_double2(a.qH, a.sig);
+      double sej = a.seps;
+      if (!UNI) {
+        j3 = e[(UNI ? 0 : 5) * kW64Ring];
+        j4 = e[(UNI ? 0 : 6) * kW64Ring];
+        sej = e[(UNI ? 0 : 7) * kW64Ring].x;
+      }
+      const double4 da = make_double4(d0.x, d0.y, d1.x, d1.y);
+      const double j1x = j0.x, j1y = j0.y, j1z = j1.x, j2x = j1.y, j2y = j2.x, j2z = j2.y;
+      const double qjO = j3.x, qj1 = j3.y, qj2 = j4.x, sgj = j4.y;
       const double r2a = da.w;
       // switch (zero width inside rc - width: s = 1 and ds = 0 exactly there)
       const double zz = fmax(r2a - a.rlo2, 0.0) * a.inv_sw;
@@ -239,19 +287,19 @@ __global__ void __launch_bounds__(kW64Warps * 32, MMNB_W64_BLOCKS) k_pair_water6
       const unsigned bal = __ballot_sync(0xffffffffu, take);
       if (take) {
         const int slot = (head + qn + __popc(bal & below)) & (kW64Ring - 1);
-        qa[slot] = make_double4(x, y, z, r2a);
-        const double4 *src = a.rec + 3 * (size_t) jc;
-        cp16(&q0[slot], src);
-        cp16(reinterpret_cast<double2 *>(&q0[slot]) + 1, reinterpret_cast<const double2 *>(src) + 1);
-        cp16(&q1[slot], src + 1);
-        cp16(reinterpret_cast<double2 *>(&q1[slot]) + 1, reinterpret_cast<const double2 *>(src + 1) + 1);
-        cp16(&q2[slot], src + 2);
-        cp16(reinterpret_cast<double2 *>(&q2[slot]) + 1, reinterpret_cast<const double2 *>(src + 2) + 1);
+        double2 *const e = q + slot;
+        e[0] = make_double2(x, y);
+        e[kW64Ring] = make_double2(z, r2a);
+        const double2 *src = a.rec + 6 * (size_t) jc;
+#pragma unroll
+        for (int k = 0; k < kWords - 2; k++)
+          cp16(e + (2 + k) * kW64Ring, src + k);
       }
       asm volatile("cp.async.commit_group;\n" ::: "memory");
       const bool run = qn >= 32;
       qn += __popc(bal);
       if (run) {
+        wait_table();
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         __syncwarp();
         compute((head + lane) & (kW64Ring - 1));
@@ -263,6 +311,7 @@ __global__ void __launch_bounds__(kW64Warps * 32, MMNB_W64_BLOCKS) k_pair_water6
       jn = jnn;
       ac = an;
     }
+    wait_table();
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncwarp();
     for (; qn > 0; qn -= 32, head = (head + 32) & (kW64Ring - 1))
@@ -271,8 +320,8 @@ __global__ void __launch_bounds__(kW64Warps * 32, MMNB_W64_BLOCKS) k_pair_water6
     // row totals: lanes' values transposed through the warp's ring, each of
     // lanes 0..15 adds one column over the 32 lanes in lane order
     __syncwarp();
-    double(*red)[kW64Acc + 1] = reinterpret_cast<double(*)[kW64Acc + 1]>(qa);
-    static_assert(32 * (kW64Acc + 1) * sizeof(double) <= 4 * kW64Ring * sizeof(double4), "ring too small");
+    double(*red)[kW64Acc + 1] = reinterpret_cast<double(*)[kW64Acc + 1]>(q);
+    static_assert(32 * (kW64Acc + 1) * sizeof(double) <= kWords * kW64Ring * sizeof(double2), "ring too small");
 #pragma unroll
     for (int c = 0; c < kW64Acc; c++)
       red[lane][c] = acc[c];
@@ -298,6 +347,7 @@ __global__ void __launch_bounds__(kW64Warps * 32, MMNB_W64_BLOCKS) k_pair_water6
     }
     __syncwarp();  // the ring is the next row's again only after every lane has read it
   }
+  wait_table();  // warps without a row meet the others here
 }
 
 // Per step: sorted FP64 anchors and the 96-byte records of the partner side,
@@ -307,7 +357,7 @@ __global__ void __launch_bounds__(kW64Warps * 32, MMNB_W64_BLOCKS) k_pair_water6
 __global__ void k_sort_water64(const double *__restrict__ r, const double *__restrict__ q,
                                const double *__restrict__ sig, const double *__restrict__ eps,
                                const int *__restrict__ sorted, const int *__restrict__ group, int ngroup,
-                               double4 *__restrict__ anchor, double4 *__restrict__ rec,
+                               double4 *__restrict__ anchor, double2 *__restrict__ rec,
                                unsigned long long *__restrict__ counter, int *__restrict__ flags)
 {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -321,64 +371,62 @@ __global__ void k_sort_water64(const double *__restrict__ r, const double *__res
   if (!isfinite(ax + ay + az + h1[0] + h1[1] + h1[2] + h2[0] + h2[1] + h2[2]))
     flags[kFlagError] = MMNB_ERR_DEVICE;
   anchor[p] = make_double4(ax, ay, az, 0.0);
-  rec[3 * (size_t) p] = make_double4(h1[0] - ax, h1[1] - ay, h1[2] - az, h2[0] - ax);
-  rec[3 * (size_t) p + 1] = make_double4(h2[1] - ay, h2[2] - az, q[a0], q[a0 + 1]);
-  rec[3 * (size_t) p + 2] = make_double4(q[a0 + 2], sig[a0], sqrt(eps[a0]), 0.0);
-}
-
-static size_t water64_smem(const mmnb_handle *h, int warps)
-{
-  return sizeof(double4) * 4 * kW64Ring * warps + sizeof(double2) * 2 * (size_t) h->cheb_w_nseg;
+  double2 *const o = rec + 6 * (size_t) p;
+  o[0] = make_double2(h1[0] - ax, h1[1] - ay);
+  o[1] = make_double2(h1[2] - az, h2[0] - ax);
+  o[2] = make_double2(h2[1] - ay, h2[2] - az);
+  o[3] = make_double2(q[a0], q[a0 + 1]);
+  o[4] = make_double2(q[a0 + 2], sig[a0]);
+  o[5] = make_double2(sqrt(eps[a0]), 0.0);
 }
 
 cudaError_t launch_sort_water64(mmnb_handle *h, const double *d_r)
 {
   k_sort_water64<<<div_up(h->ngroup, 256), 256, 0, h->stream>>>(
-      d_r, h->d_q, h->d_sig, h->d_eps, h->d_sorted, h->d_group, h->ngroup, h->d_sp, h->d_sr, h->d_wsum + 3,
+      d_r, h->d_q, h->d_sig, h->d_eps, h->d_sorted, h->d_group, h->ngroup, h->d_sp, reinterpret_cast<double2 *>(h->d_sr), h->d_wsum + 3,
       h->d_flags);
+  h->launches += 1;
+  return cudaGetLastError();
+}
+
+template <bool VIR, bool UNI>
+static cudaError_t launch_water64(mmnb_handle *h, Water64Args &a)
+{
+  cudaError_t e;
+  int optin = 0, nsm = 0;
+  if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->dev)) != cudaSuccess ||
+      (e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->dev)) != cudaSuccess)
+    return e;
+  // the tuned warps per block, fewer if the rings and this box's table do not fit
+  // (the table grows as rc falls)
+  const size_t ring = sizeof(double2) * w64_words(UNI) * kW64Ring, table = sizeof(double2) * 2 * (size_t) a.nseg;
+  // (and on a small box no more than it takes to cover the SMs: a block's warps
+  // share one SM's pipes)
+  int warps = std::min(std::min(h->tune.water64_warps, kW64Warps), std::max(4, (div_up(h->ngroup, nsm) + 1) / 2 * 2));
+  while (warps > 4 && ring * warps + table > (size_t) optin)
+    warps -= 2;
+  // as many copies of the table as fit, where a warp takes enough rows to fill
+  // them for (below about two, one copy)
+  a.copies = (long) h->ngroup >= 2L * nsm * warps ? 8 : 1;
+  while (a.copies > 1 && ring * warps + table * a.copies > (size_t) optin)
+    a.copies >>= 1;
+  if ((e = cudaFuncSetAttribute(k_pair_water64<VIR, UNI>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin)) !=
+      cudaSuccess)
+    return e;
+  k_pair_water64<VIR, UNI><<<std::min(nsm, div_up(h->ngroup, warps)), 32 * warps, ring * warps + table * a.copies,
+                             h->stream>>>(a);
   h->launches += 1;
   return cudaGetLastError();
 }
 
 cudaError_t launch_rspace_water64(mmnb_handle *h)
 {
-  cudaError_t e;
-  int optin = 0;
-  if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->dev)) != cudaSuccess)
-    return e;
-  // the tuned warps per block, fewer if the rings and this box's table do not
-  // fit (the table grows with rc: 12 warps below ~22 KB of table)
-  int warps = std::min(h->tune.water64_warps, kW64Warps);
-  while (warps > 4 && water64_smem(h, warps) > (size_t) optin)
-    warps -= 2;
-  if (h->water64_grid == 0 || warps != h->water64_warps) {
-    int nsm = 0;
-    if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->dev)) != cudaSuccess)
-      return e;
-    const size_t smem = water64_smem(h, warps);
-    if ((e = cudaFuncSetAttribute(k_pair_water64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) !=
-            cudaSuccess ||
-        (e = cudaFuncSetAttribute(k_pair_water64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) !=
-            cudaSuccess)
-      return e;
-    int per_sm = 0, per_sm_v = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_water64<false>, warps * 32, smem)) !=
-            cudaSuccess ||
-        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_v, k_pair_water64<true>, warps * 32, smem)) !=
-            cudaSuccess)
-      return e;
-    per_sm = std::min(per_sm, per_sm_v);
-    if (per_sm < 1)
-      return cudaErrorLaunchOutOfResources;
-    h->water64_grid = std::min(per_sm * nsm, div_up(h->ngroup, warps));
-    h->water64_smem = smem;
-    h->water64_warps = warps;
-  }
   Water64Args a;
   a.ngroup = h->ngroup;
   a.rowcap = h->rowcap;
   a.geometric = h->cfg.geometric_combining_for_sigma;
   a.nseg = h->cheb_w_nseg;
+  a.series = h->eta * sqrt(h->cheb_min) <= kErfSeriesMax;
   a.box = h->box;
   a.rlo2 = h->rlo2;
   a.rhi2 = h->rhi2;
@@ -387,10 +435,14 @@ cudaError_t launch_rspace_water64(mmnb_handle *h)
   a.cmin = h->cheb_min;
   a.inv_dx = h->cheb_inv_dx;
   a.dscale = -2 * h->cheb_inv_dx;
-  a.nsegd = (double) h->cheb_w_nseg;
+  a.nsegd = table_segments(h);
   a.table = reinterpret_cast<const double2 *>(h->d_cheb_w);
   a.anchor = h->d_sp;
-  a.rec = h->d_sr;
+  a.rec = reinterpret_cast<const double2 *>(h->d_sr);
+  a.qO = h->uni64[0];
+  a.qH = h->uni64[1];
+  a.sig = h->uni64[2];
+  a.seps = h->uni64[3];
   a.nbr = h->d_nbr;
   a.nbr_count = h->d_nbr_count;
   a.sorted = h->d_sorted;
@@ -403,11 +455,8 @@ cudaError_t launch_rspace_water64(mmnb_handle *h)
   a.vir_row = h->want_virial ? h->d_vir_row : nullptr;
   a.cheb_d = h->d_cheb_d;
   if (h->want_virial)
-    k_pair_water64<true><<<h->water64_grid, h->water64_warps * 32, h->water64_smem, h->stream>>>(a);
-  else
-    k_pair_water64<false><<<h->water64_grid, h->water64_warps * 32, h->water64_smem, h->stream>>>(a);
-  h->launches += 1;
-  return cudaGetLastError();
+    return h->water_uni ? launch_water64<true, true>(h, a) : launch_water64<true, false>(h, a);
+  return h->water_uni ? launch_water64<false, true>(h, a) : launch_water64<false, false>(h, a);
 }
 
 }  // namespace mmnb

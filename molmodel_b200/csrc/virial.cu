@@ -173,7 +173,7 @@ extern "C" int mmnb_virial(mmnb_handle *h, const double *r, int nmol, const int 
   int npart = 0;
   const unsigned long long *fixed = nullptr;
   if (h->cfg.include_rspace) {
-    if (h->used_water64) {
+    if (h->used_rows64) {
       part = h->d_vir_row;
       npart = h->ngroup;
     } else if (h->used_water) {
