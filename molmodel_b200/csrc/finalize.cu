@@ -192,13 +192,13 @@ cudaError_t launch_finalize(mmnb_handle *h, double *d_f, double *d_energy)
   a.lj_part = h->d_lj_part;
   // the water kernel leaves its LJ energy in the fixed-point word, not in the
   // pair partials
-  a.lj_lo = (h->used_water || h->used_rows64) ? h->lj_pair_blocks : 0;
+  a.lj_lo = (h->used_fx || h->used_rows64) ? h->lj_pair_blocks : 0;
   a.lj_row = h->used_rows64 ? h->d_lj_row : nullptr;
   a.nrow = h->ngroup;
   a.lj_row_part = h->d_lj_row_part;
   a.lj_hi = h->lj_pair_blocks + h->lj_excl_blocks;
   a.any_q = h->any_q ? 1 : 0;
-  a.wsum = h->used_water ? h->d_wsum : nullptr;
+  a.wsum = h->used_fx ? h->d_wsum : nullptr;
   a.counter = h->d_wsum + 2;
   a.flags = h->d_flags;
   a.tail = h->cfg.include_lj_correction ? h->lj_correction : 0.0;

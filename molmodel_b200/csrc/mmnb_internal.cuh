@@ -124,7 +124,7 @@ struct mmnb_handle {
   double uni64[4] = {0, 0, 0, 0};    // the same in FP64
   bool want_fields = false;          // this evaluation must produce per-site potential and field
   bool want_virial = false;          // this evaluation's pair kernels also sum the virial's pair term
-  bool used_water = false;           // the last evaluation ran the water kernel
+  bool used_fx = false;              // the last evaluation ran a mixed pair kernel: fixed-point energies
   bool used_rows64 = false;          // the last evaluation ran an FP64 pair kernel: energies per row
   double totA = 0, totB = 0, lj_correction = 0, neutral_b = 0;
 
@@ -209,9 +209,9 @@ struct mmnb_handle {
   int *d_vir_mol = nullptr;
   double *d_vir_molw = nullptr, *d_vir_mass = nullptr;
   int vir_mol_cap = 0;
-  // [0], [1]: fixed-point Coulomb and LJ pair energies of the water kernel;
+  // [0], [1]: fixed-point Coulomb (rigid water) and LJ pair energies of the mixed pair kernels;
   // [2]: block counter of the finalize kernel's last-block reduction;
-  // [3]: row counter of the FP64 water kernel; [4]: the mixed water kernel's
+  // [3]: row counter of the FP64 pair kernels; [4]: the mixed pair kernels'
   // fixed-point virial term
   unsigned long long *d_wsum = nullptr;
   // parameter gradients (allocated on first use): six per-site outputs, dL/dF

@@ -32,10 +32,10 @@
 //     the term, so the sums of a lane are one site's: 12 doubles at most, and the
 //     kernel is the same for groups of one site and of eight.
 // The reference's table (continued past 1.2 rc^2 by segments of the same
-// construction where table_segments allows it) is in shared memory, the cubic alone: b1 is -2 / dx times its derivative, which is how
-// the reference stores it; below the table (r^2 < 4) ewald_short.  Lanes' sums are
-// added in a fixed order: no atomics, bitwise reproducible whichever warp takes a
-// row.
+// construction where table_segments allows it) is in shared memory, the cubic
+// alone: b1 is -2 / dx times its derivative, which is how the reference stores it;
+// below the table (r^2 < 4) ewald_short.  Lanes' sums are added in a fixed order:
+// no atomics, bitwise reproducible whichever warp takes a row.
 //
 // Bound by latency (12 warps of 168 registers per SM; 16 of 128 spill and were
 // slower, 86 against 115 us) and the shared-memory pipe.  Measured on 17^3 cells of

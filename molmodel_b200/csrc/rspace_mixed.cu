@@ -13,24 +13,30 @@
 //     relative accuracy (below), exp(-eta^2 r^2) shared with the field term
 //     b1 = (b0 + 2 eta/sqrt(pi) exp(-eta^2 r^2)) / r^2;
 //   * the switch and LJ terms are the FP64 form's formulas in FP32.
-// Each group pair's contribution to each row site (potential, field, LJ
+// A partner group's contribution to each row site (potential, field, LJ
 // force) is summed in FP32 and then converted to 64-bit fixed point
 // (2^32 units per unit) before it is added: integer addition is associative,
 // so the totals do not depend on the list order, on which lane took which
 // pair, or on the reduction order — the forces are bitwise deterministic.
 //
-// Work layout as in the FP64 form: full list, one warp per row group, a
-// ballot-compacted shared-memory queue of in-cutoff partners so every lane
-// evaluates a group pair, and a shared-memory transpose to reduce the lanes'
-// fixed-point totals.
+// Work layout: full list, one warp per row group, partners inside the cutoff
+// ballot-compacted into a queue in shared memory.  A lane takes one site of the
+// row and one queued partner (32 / n partners per step for a row of n sites) and
+// walks the partner's sites, so it holds one site's sums whatever the groups'
+// size and registers leave room for 20 warps per SM, which is what hides the
+// partners' record loads.  Only the switch derivative needs the whole group pair:
+// its unswitched energy is summed over the row sites' lanes by shuffles.
+//
+// A lane per partner group over all its padded site pairs, with 7 x 4 64-bit sums
+// and an exclusion search per group pair: 494 us on 32^3 cells of solution (94,000
+// sites, groups of two to four); this layout 260 us (bound by issue, 63%; 290 us at 16 warps per SM, 260 at 24 with spills).
 
 #include "mmnb_internal.cuh"
 
 namespace mmnb {
 
-constexpr int kMxWarps = 4;
-constexpr int kMxQueue = 64;
-constexpr int kNacc = 7;  // phi, E (3), LJ force (3)
+constexpr int kMxQueue = 64;  // at most 31 carried over and 32 new
+constexpr int kNacc = 7;      // phi, E (3), LJ force (3)
 
 // erfc(x) ~= t P(t) exp(-x^2), t = 1/(1 + p x): Hastings' form (Abramowitz &
 // Stegun 7.1.26) with P refitted for relative accuracy (<= 4e-7 for all x >= 0,
@@ -88,87 +94,102 @@ struct MixedArgs {
   float rlo2, inv_sw, eta, c2, nel2;  // c2 = 2 eta / sqrt(pi), nel2 = -eta^2 log2(e)
   const float4 *site;           // offset from anchor, charge
   const float4 *par;            // sigma, sqrt(eps), rscreen, mask bits
-  const double4 *anchor;
-  const int *nbr, *nbr_count, *sorted, *group;
+  const double4 *anchor;        // sorted groups: anchor, packed first site and site masks
+  const int *nbr, *nbr_count, *sorted;
   const int *gexcl_ptr, *gexcl_idx, *excl_ptr, *excl_idx;
   long long *acc;               // per site, kAccStride
-  double *lj_part;
-  double *vir_part;             // per block: the virial's pair term (mmnb_virial), or null
+  unsigned long long *wsum;     // [1]: fixed-point LJ energy, [4]: the virial's pair term
 };
 
 __device__ __forceinline__ long long to_fx(float v) { return __float2ll_rn(v * 4294967296.0f); }
 
-// one group pair inside the cutoff: FP32 sums, then fixed point
-template <int G, bool SCREEN, bool GEXCL, bool ANCHOR_LJ>
-__device__ __forceinline__ void pair_mixed(const MixedArgs &a, const float4 (&oi)[G], const float4 (&pi)[G], int gi,
-                                           int si0, int q, float4 da, long long (&fx)[G][kNacc], long long &fe,
-                                           long long &fv)
+// G: slots per group (sites padded)
+template <int G, bool SCREEN, bool GEXCL, bool VIR>
+__global__ void __launch_bounds__(32, 20) k_pair_mixed(MixedArgs a)
 {
-  float4 oj[G], pj[G];
-#pragma unroll
-  for (int k = 0; k < G; k++) {
-    oj[k] = a.site[(size_t) q * G + k];
-    pj[k] = a.par[(size_t) q * G + k];
-  }
-  const float r2a = da.w;
-  float s = 1.f, ds = 0.f;
-  const bool smoothing = r2a > a.rlo2;
-  if (smoothing) {
-    const float z = (r2a - a.rlo2) * a.inv_sw;
-    s = fmaf(fmaf(fmaf(-6.f, z, 15.f), z, -10.f), z * z * z, 1.f);
-    ds = fmaf(fmaf(60.f, z, -120.f), z, 60.f) * z * z * a.inv_sw;
-  }
-  bool gx = false;
-  int sj0 = 0;
+  constexpr int kMask = kMxQueue - 1, kVals = kNacc + (VIR ? 2 : 1);
+  __shared__ float4 qda[kMxQueue];   // anchor displacement and r^2
+  __shared__ int qj[kMxQueue], qm[kMxQueue], qs[GEXCL ? kMxQueue : 1];
+  __shared__ long long red[32][kVals | 1];
+  const int lane = threadIdx.x & 31;
+  const int p = blockIdx.x;
+  const double4 ai = a.anchor[p];
+  const long long info = __double_as_longlong(ai.w);
+  const int si0 = (int) (info >> 32), mi = (int) info, ns = mi & 0xff;
+  const int cnt = a.nbr_count[p];
+  const int *row = a.nbr + (size_t) p * a.rowcap;
+  // entries past the row end read the row's own group (a valid address)
+  int jc = lane < cnt ? row[lane] : p;
+  int jn = lane + 32 < cnt ? row[lane + 32] : p;
+  double4 ac = a.anchor[jc];
+  const int P = 32 / ns, ia = lane / P, pk = lane - ia * P;
+  const bool act = ia < ns;
+  const float4 oi = a.site[(size_t) p * G + (act ? ia : 0)], pi = a.par[(size_t) p * G + (act ? ia : 0)];
+  const bool qi = act && (mi >> (8 + ia)) & 1, li = act && (mi >> (16 + ia)) & 1;
+  int gi = 0;
+  bool row_gx = false;
   if (GEXCL) {
-    const int gj = a.sorted[q];
-    gx = csr_has(a.gexcl_ptr, a.gexcl_idx, gi, gj);
-    sj0 = a.group[2 * gj];
+    gi = a.sorted[p];
+    row_gx = a.gexcl_ptr[gi + 1] > a.gexcl_ptr[gi];
   }
-  float ph[G], ex[G], ey[G], ez[G], lx[G], ly[G], lz[G];
+  const unsigned below = (1u << lane) - 1;
+  long long fx[kNacc] = {0, 0, 0, 0, 0, 0, 0}, fe = 0, fv = 0;
+  int head = 0, qn = 0;
+  // row site ia against the queued partner pk, n queued
+  auto eval = [&](int n) {
+    const bool live = act && pk < n;
+    const int k = (head + pk) & kMask;
+    const float4 da = qda[k];
+    const int q = qj[k], mj = live ? qm[k] : 0, nsj = mj & 0xff;
+    float4 oj[G];
 #pragma unroll
-  for (int k = 0; k < G; k++)
-    ph[k] = ex[k] = ey[k] = ez[k] = lx[k] = ly[k] = lz[k] = 0.f;
-  float tmps = 0.f, u_sum = 0.f, xv = 0.f;
-#pragma unroll
-  for (int ia = 0; ia < G; ia++) {
-    const int mi = __float_as_int(pi[ia].w);
-    const float cx = da.x + oi[ia].x, cy = da.y + oi[ia].y, cz = da.z + oi[ia].z;
-    float tq = 0.f;  // sum_j q_j b0 before switching, for the switch derivative
+    for (int jb = 0; jb < G; jb++)
+      if (jb < nsj)
+        oj[jb] = a.site[(size_t) q * G + jb];
+    const float z = fmaxf(da.w - a.rlo2, 0.f) * a.inv_sw;
+    const float s = fmaf(fmaf(fmaf(-6.f, z, 15.f), z, -10.f), z * z * z, 1.f);
+    const float ds = fmaf(fmaf(60.f, z, -120.f), z, 60.f) * z * z * a.inv_sw;
+    const bool gx = GEXCL && row_gx && (mj >> 24) & 1;
+    const float cx = da.x + oi.x, cy = da.y + oi.y, cz = da.z + oi.z;
+    float ph = 0.f, ex = 0.f, ey = 0.f, ez = 0.f, lx = 0.f, ly = 0.f, lz = 0.f;
+    float tq = 0.f, tu = 0.f, us = 0.f, xv = 0.f;  // sum q_j b0 and LJ energies before the switch, switched LJ
 #pragma unroll
     for (int jb = 0; jb < G; jb++) {
-      const int m = mi & __float_as_int(pj[jb].w);
-      if (!m)
+      if (jb >= nsj)
+        break;
+      const bool hq = qi && (mj >> (8 + jb)) & 1, hl = li && (mj >> (16 + jb)) & 1;
+      if (!hq && !hl)
         continue;
-      if (GEXCL && gx && csr_has(a.excl_ptr, a.excl_idx, si0 + ia, sj0 + jb))
+      if (GEXCL && gx && csr_has(a.excl_ptr, a.excl_idx, si0 + ia, qs[GEXCL ? k : 0] + jb))
         continue;
       const float dx = cx - oj[jb].x, dy = cy - oj[jb].y, dz = cz - oj[jb].z;
       const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
       const float rinv = rsqrt_approx(r2);
-      if (m & MMNB_SITE_HAS_Q) {
+      if (hq) {
         float b0, b1;
         ewald_f32(r2, rinv, a.eta, a.nel2, a.c2, b0, b1);
         if (SCREEN) {
-          const float rs = pi[ia].z + pj[jb].z;
+          const float rs = pi.z + a.par[(size_t) q * G + jb].z;
           if (r2 < rs * rs) {
             const float inv3 = 1.f / (rs * rs * rs);
             b0 += fmaf(-0.5f * r2, inv3, 1.5f / rs) - rinv;
             b1 += inv3 - rinv * rinv * rinv;
           }
         }
-        const float qj = oj[jb].w;
-        tq = fmaf(qj, b0, tq);
-        const float qs = qj * s;
-        ph[ia] = fmaf(qs, b0, ph[ia]);
-        const float f = qs * b1;
-        ex[ia] = fmaf(f, dx, ex[ia]);
-        ey[ia] = fmaf(f, dy, ey[ia]);
-        ez[ia] = fmaf(f, dz, ez[ia]);
+        const float qjv = oj[jb].w;
+        tq = fmaf(qjv, b0, tq);
+        const float qs1 = qjv * s;
+        ph = fmaf(qs1, b0, ph);
+        const float f = qs1 * b1;
+        ex = fmaf(f, dx, ex);
+        ey = fmaf(f, dy, ey);
+        ez = fmaf(f, dz, ez);
       }
-      if (m & MMNB_SITE_HAS_LJ) {
-        const float sg = a.geometric ? pi[ia].x * pj[jb].x : 0.5f * (pi[ia].x + pj[jb].x) * 0.5f * (pi[ia].x + pj[jb].x);
+      if (hl) {
+        const float4 pj = a.par[(size_t) q * G + jb];
+        const float sg = a.geometric ? pi.x * pj.x : 0.5f * (pi.x + pj.x) * 0.5f * (pi.x + pj.x);
         const float s6 = sg * sg * sg;
-        const float b = 4.f * pi[ia].y * pj[jb].y * s6;
+        const float b = 4.f * pi.y * pj.y * s6;
         const float aa = b * s6;
         const float ir2 = rinv * rinv;
         const float ir6 = ir2 * ir2 * ir2;
@@ -176,165 +197,98 @@ __device__ __forceinline__ void pair_mixed(const MixedArgs &a, const float4 (&oi
         const float ai12 = aa * ir6 * ir6;
         const float du = (12.f * ai12 - 6.f * bi6) * ir2 * s;
         const float u = ai12 - bi6;
-        tmps += u;
-        u_sum = fmaf(u, s, u_sum);
-        xv = fmaf(du, r2, xv);
-        lx[ia] = fmaf(du, dx, lx[ia]);
-        ly[ia] = fmaf(du, dy, ly[ia]);
-        lz[ia] = fmaf(du, dz, lz[ia]);
+        tu += u;
+        us = fmaf(u, s, us);
+        if (VIR)
+          xv = fmaf(du, r2, xv);
+        lx = fmaf(du, dx, lx);
+        ly = fmaf(du, dy, ly);
+        lz = fmaf(du, dz, lz);
       }
     }
-    tmps = fmaf(oi[ia].w, tq, tmps);
-  }
-  if (smoothing) {
-    const float g = ds * tmps;
-    lx[0] = fmaf(g, da.x, lx[0]);
-    ly[0] = fmaf(g, da.y, ly[0]);
-    lz[0] = fmaf(g, da.z, lz[0]);
-    xv = fmaf(g, r2a, xv);
-  }
-#pragma unroll
-  for (int k = 0; k < G; k++) {
-    fx[k][0] += to_fx(ph[k]);
-    fx[k][1] += to_fx(ex[k]);
-    fx[k][2] += to_fx(ey[k]);
-    fx[k][3] += to_fx(ez[k]);
-    if (!ANCHOR_LJ || k == 0) {
-      fx[k][4] += to_fx(lx[k]);
-      fx[k][5] += to_fx(ly[k]);
-      fx[k][6] += to_fx(lz[k]);
+    // the group pair's unswitched energy, over the row sites' lanes
+    const float e = fmaf(oi.w, tq, tu);
+    float et = e;
+    for (int o = 1; o < ns; o++)
+      et += __shfl_down_sync(0xffffffffu, e, o * P);
+    if (ia == 0) {
+      const float g = ds * et;
+      lx = fmaf(g, da.x, lx);
+      ly = fmaf(g, da.y, ly);
+      lz = fmaf(g, da.z, lz);
+      if (VIR)
+        xv = fmaf(g, da.w, xv);
     }
-  }
-  fe += to_fx(0.5f * u_sum);
-  if (a.vir_part)
-    fv += to_fx(0.5f * xv);
-}
-
-template <int G, bool SCREEN, bool GEXCL, bool ANCHOR_LJ>
-__global__ void __launch_bounds__(kMxWarps * 32) k_pair_mixed(MixedArgs a)
-{
-  __shared__ float4 qda[kMxWarps][kMxQueue];
-  __shared__ int qix[kMxWarps][kMxQueue];
-  constexpr int kCols = G * kNacc + 2;  // site values, LJ energy, virial term
-  constexpr bool kTranspose = G <= 4;
-  __shared__ long long red[kTranspose ? kMxWarps : 1][kTranspose ? 32 : 1][kTranspose ? kCols : 1];
-  __shared__ long long wlj[kMxWarps], wvir[kMxWarps];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int p = blockIdx.x * kMxWarps + w;
-  long long fx[G][kNacc];
-#pragma unroll
-  for (int k = 0; k < G; k++)
-#pragma unroll
-    for (int c = 0; c < kNacc; c++)
-      fx[k][c] = 0;
-  long long fe = 0, fv = 0;
-  int gi = 0, si0 = 0, ns = 0;
-  if (p < a.ngroup) {
-    float4 oi[G], pi[G];
-#pragma unroll
-    for (int k = 0; k < G; k++) {
-      oi[k] = a.site[(size_t) p * G + k];
-      pi[k] = a.par[(size_t) p * G + k];
+    if (live) {
+      fx[0] += to_fx(ph);
+      fx[1] += to_fx(ex);
+      fx[2] += to_fx(ey);
+      fx[3] += to_fx(ez);
+      fx[4] += to_fx(lx);
+      fx[5] += to_fx(ly);
+      fx[6] += to_fx(lz);
+      fe += to_fx(0.5f * us);
+      if (VIR)
+        fv += to_fx(0.5f * xv);
     }
-    const double4 ai = a.anchor[p];
-    gi = a.sorted[p];
-    si0 = a.group[2 * gi];
-    ns = a.group[2 * gi + 1] - si0;
-    const int cnt = a.nbr_count[p];
-    const int *row = a.nbr + (size_t) p * a.rowcap;
-    const unsigned below = (1u << lane) - 1;
-    int qn = 0;
-    for (int base = 0; base < cnt; base += 32) {
-      const int e = base + lane;
-      bool take = false;
-      int q = 0;
-      float4 da = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (e < cnt) {
-        q = row[e];
-        double x, y, z, sx, sy, sz;
-        const double r2a = anchor_disp(a.box, ai, a.anchor[q], x, y, z, sx, sy, sz);
-        take = r2a <= a.rhi2;
-        da = make_float4((float) x, (float) y, (float) z, (float) r2a);
+    head = (head + n) & kMask;
+    qn -= n;
+    __syncwarp();  // the slots are free again only after every lane has read them
+  };
+  for (int base = 0; base < cnt; base += 32) {
+    const int e2 = base + 64 + lane;
+    const int jnn = e2 < cnt ? row[e2] : p;
+    const double4 an = a.anchor[jn];
+    double x, y, z, sx, sy, sz;
+    const double r2a = anchor_disp(a.box, ai, ac, x, y, z, sx, sy, sz);
+    const bool take = base + lane < cnt && r2a <= a.rhi2;
+    const unsigned bal = __ballot_sync(0xffffffffu, take);
+    if (take) {
+      const int k = (head + qn + __popc(bal & below)) & kMask;
+      qda[k] = make_float4((float) x, (float) y, (float) z, (float) r2a);
+      qj[k] = jc;
+      const long long ij = __double_as_longlong(ac.w);
+      int m = (int) ij;
+      if (GEXCL && row_gx) {
+        qs[GEXCL ? k : 0] = (int) (ij >> 32);
+        if (csr_has(a.gexcl_ptr, a.gexcl_idx, gi, a.sorted[jc]))
+          m |= 1 << 24;
       }
-      const unsigned bal = __ballot_sync(0xffffffffu, take);
-      if (take) {
-        const int idx = qn + __popc(bal & below);
-        qda[w][idx] = da;
-        qix[w][idx] = q;
-      }
-      qn += __popc(bal);
-      __syncwarp();
-      if (qn >= 32) {
-        pair_mixed<G, SCREEN, GEXCL, ANCHOR_LJ>(a, oi, pi, gi, si0, qix[w][lane], qda[w][lane], fx, fe, fv);
-        __syncwarp();
-        if (lane < qn - 32) {
-          qda[w][lane] = qda[w][lane + 32];
-          qix[w][lane] = qix[w][lane + 32];
-        }
-        __syncwarp();
-        qn -= 32;
-      }
+      qm[k] = m;
     }
-    if (lane < qn)
-      pair_mixed<G, SCREEN, GEXCL, ANCHOR_LJ>(a, oi, pi, gi, si0, qix[w][lane], qda[w][lane], fx, fe, fv);
-  }
-  if constexpr (kTranspose) {
-    // transpose reduction: lane c sums column c over the 32 lanes
-#pragma unroll
-    for (int k = 0; k < G; k++)
-#pragma unroll
-      for (int c = 0; c < kNacc; c++)
-        red[w][lane][k * kNacc + c] = fx[k][c];
-    red[w][lane][G * kNacc] = fe;
-    red[w][lane][G * kNacc + 1] = fv;
+    qn += __popc(bal);
     __syncwarp();
-    for (int c = lane; c < kCols; c += 32) {
-      long long t = 0;
-      for (int l = 0; l < 32; l++)
-        t += red[w][l][c];
-      if (c == G * kNacc) {
-        wlj[w] = t;
-      } else if (c == G * kNacc + 1) {
-        wvir[w] = t;
-      } else if (p < a.ngroup) {
-        const int k = c / kNacc, comp = c % kNacc;
-        if (k < ns)
-          a.acc[(size_t) (si0 + k) * kAccStride + comp] = t;
-      }
-    }
-  } else {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-      for (int k = 0; k < G; k++)
-#pragma unroll
-        for (int c = 0; c < kNacc; c++)
-          fx[k][c] += __shfl_xor_sync(0xffffffffu, fx[k][c], off);
-      fe += __shfl_xor_sync(0xffffffffu, fe, off);
-      fv += __shfl_xor_sync(0xffffffffu, fv, off);
-    }
-    if (lane == 0) {
-      wlj[w] = fe;
-      wvir[w] = fv;
-    }
-    if (p < a.ngroup)
-#pragma unroll
-      for (int k = 0; k < G; k++)
-        if (lane == k && k < ns)
-#pragma unroll
-          for (int c = 0; c < kNacc; c++)
-            a.acc[(size_t) (si0 + k) * kAccStride + c] = fx[k][c];
+    while (qn >= P)
+      eval(P);
+    jc = jn;
+    jn = jnn;
+    ac = an;
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    long long t = 0, v = 0;
-    for (int k = 0; k < kMxWarps; k++) {
-      t += wlj[k];
-      v += wvir[k];
-    }
-    a.lj_part[blockIdx.x] = (double) t * kFxInv;
-    if (a.vir_part)
-      a.vir_part[blockIdx.x] = (double) v * kFxInv;
+  if (qn > 0)
+    eval(qn);
+#pragma unroll
+  for (int c = 0; c < kNacc; c++)
+    red[lane][c] = fx[c];
+  red[lane][kNacc] = fe;
+  if (VIR)
+    red[lane][kVals - 1] = fv;
+  __syncwarp();
+  for (int t = lane; t < kNacc * ns; t += 32) {
+    const int i = t / kNacc, c = t - kNacc * i;
+    long long sum = 0;
+    for (int l = i * P; l < (i + 1) * P; l++)
+      sum += red[l][c];
+    a.acc[(size_t) (si0 + i) * kAccStride + c] = sum;
+  }
+  // integer sums: the totals do not depend on the order rows finish in
+#pragma unroll
+  for (int c = kNacc; c < kVals; c++) {
+    long long sum = red[lane][c];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane == 0)
+      atomicAdd(a.wsum + (c == kNacc ? 1 : 4), (unsigned long long) sum);
   }
 }
 
@@ -857,7 +811,7 @@ __device__ __forceinline__ void water_row_store_shfl(const WaterArgs &a, int si0
 // VIR: also the part of dU/ds (box scaling) the site forces do not carry, the
 // anchor force scalar times R^2 per group pair (mmnb_virial)
 template <int MINB, bool VIR, bool UNI>
-__global__ void __launch_bounds__(kWaterWarps * 32, MINB * kMxWarps / kWaterWarps) k_pair_water(WaterArgs a)
+__global__ void __launch_bounds__(kWaterWarps * 32, MINB * 4 / kWaterWarps) k_pair_water(WaterArgs a)
 {
   // per warp: ring of anchor displacement (xyz, r^2) and the partner's three
   // packed slots
@@ -980,8 +934,18 @@ __global__ void k_prep_mixed(const double *__restrict__ r, const double *__restr
   const int g = sorted[p];
   const int a0 = group[2 * g];
   const double ax = r[3 * a0], ay = r[3 * a0 + 1], az = r[3 * a0 + 2];
-  if (k == 0)
-    anchor[p] = make_double4(ax, ay, az, 0.0);
+  if (k == 0) {
+    // the group's first site (high word), number of sites, charged sites and LJ
+    // sites (a byte each of the low word: bit j for site j)
+    const int n = group[2 * g + 1] - a0;
+    unsigned m = n;
+    if (!water)
+      for (int j = 0; j < n; j++) {
+        const int b = mask[a0 + j];
+        m |= (b & MMNB_SITE_HAS_Q ? 1u << (8 + j) : 0u) | (b & MMNB_SITE_HAS_LJ ? 1u << (16 + j) : 0u);
+      }
+    anchor[p] = make_double4(ax, ay, az, __longlong_as_double((long long) a0 << 32 | m));
+  }
   // a non-finite coordinate is flagged (the host reports it); every index
   // below stays in range whatever the coordinates
   if (a0 + k < group[2 * g + 1] &&
@@ -1044,23 +1008,16 @@ cudaError_t launch_prep_mixed(mmnb_handle *h, const double *d_r)
   return cudaGetLastError();
 }
 
-template <int G, bool ANCHOR_LJ>
+template <int G>
 static void launch_mixed_g(mmnb_handle *h, const MixedArgs &a)
 {
-  const int blocks = pair_blocks(h);
-  const int threads = kMxWarps * 32;
   h->launches += 1;
-  if (h->has_rscreen) {
-    if (h->any_gexcl)
-      k_pair_mixed<G, true, true, ANCHOR_LJ><<<blocks, threads, 0, h->stream>>>(a);
-    else
-      k_pair_mixed<G, true, false, ANCHOR_LJ><<<blocks, threads, 0, h->stream>>>(a);
-  } else {
-    if (h->any_gexcl)
-      k_pair_mixed<G, false, true, ANCHOR_LJ><<<blocks, threads, 0, h->stream>>>(a);
-    else
-      k_pair_mixed<G, false, false, ANCHOR_LJ><<<blocks, threads, 0, h->stream>>>(a);
-  }
+  auto *k = h->want_virial  // (mmnb_virial refuses screened charges)
+                ? (h->any_gexcl ? k_pair_mixed<G, false, true, true> : k_pair_mixed<G, false, false, true>)
+            : h->has_rscreen
+                ? (h->any_gexcl ? k_pair_mixed<G, true, true, false> : k_pair_mixed<G, true, false, false>)
+                : (h->any_gexcl ? k_pair_mixed<G, false, true, false> : k_pair_mixed<G, false, false, false>);
+  k<<<h->ngroup, 32, 0, h->stream>>>(a);
 }
 
 cudaError_t launch_rspace_mixed(mmnb_handle *h)
@@ -1082,21 +1039,18 @@ cudaError_t launch_rspace_mixed(mmnb_handle *h)
   a.nbr = h->d_nbr;
   a.nbr_count = h->d_nbr_count;
   a.sorted = h->d_sorted;
-  a.group = h->d_group;
   a.gexcl_ptr = h->d_gexcl_ptr;
   a.gexcl_idx = h->d_gexcl_idx;
   a.excl_ptr = h->d_excl_ptr;
   a.excl_idx = h->d_excl_idx;
   a.acc = h->mx.acc;
-  a.lj_part = h->d_lj_part;
-  a.vir_part = h->want_virial ? h->d_vir_part : nullptr;
-  const bool alj = h->lj_on_anchors_only;
+  a.wsum = h->d_wsum;
   switch (h->G) {
-  case 1: launch_mixed_g<1, false>(h, a); break;
-  case 2: alj ? launch_mixed_g<2, true>(h, a) : launch_mixed_g<2, false>(h, a); break;
-  case 3: alj ? launch_mixed_g<3, true>(h, a) : launch_mixed_g<3, false>(h, a); break;
-  case 4: alj ? launch_mixed_g<4, true>(h, a) : launch_mixed_g<4, false>(h, a); break;
-  default: launch_mixed_g<8, false>(h, a); break;
+  case 1: launch_mixed_g<1>(h, a); break;
+  case 2: launch_mixed_g<2>(h, a); break;
+  case 3: launch_mixed_g<3>(h, a); break;
+  case 4: launch_mixed_g<4>(h, a); break;
+  default: launch_mixed_g<8>(h, a); break;
   }
   return cudaGetLastError();
 }

@@ -176,7 +176,7 @@ extern "C" int mmnb_virial(mmnb_handle *h, const double *r, int nmol, const int 
     if (h->used_rows64) {
       part = h->d_vir_row;
       npart = h->ngroup;
-    } else if (h->used_water) {
+    } else if (h->used_fx) {
       fixed = h->d_wsum + 4;
     } else {
       npart = h->lj_pair_blocks;

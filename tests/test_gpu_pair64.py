@@ -1,10 +1,11 @@
-"""The FP64 pair kernel for groups of any size, at the group sizes, row counts and
-screening parameters where its queues, teams of warps and short-range branch can
-go wrong, against the oracle (1e-10, the FP64 form's bound)."""
+"""The pair kernels for groups of any size, at the group sizes, row counts and
+screening parameters where their queues, teams of warps and short-range branch can
+go wrong, against the oracle (FP64 form: 1e-10; mixed form: 1e-5 RMS, both the
+forms' bounds)."""
 import numpy as np
 import pytest
 
-from conftest import rel_max
+from conftest import rel_max, rel_rms
 from molmodel_b200 import ElecLJ, water_box_n
 from oracle.oracle import make_config, port
 
@@ -88,3 +89,22 @@ def test_rigid_water(eta, uniform):
     if not uniform:
         S.q[0] *= 1.01
     check(S, ewald_screening=eta)
+
+
+@pytest.mark.parametrize("sizes", [(1,), (2,), (1, 2, 3), (4, 1), (5, 3), (8,), (7, 1, 8, 2)])
+def test_mixed_group_sizes(sizes):
+    s = Grouped(216, sizes, seed=sum(sizes))
+    s.rscreen = np.where(np.arange(s.nsite) % 5 == 0, 1.5, 0.0)
+    cfg = dict(rspace_cutoff=7.0, ewald_screening=0.4, kspace_cutoff=4.0)
+    o = port().eleclj(make_config(s.box, **cfg), s.nsite, s.groups, s.exclusions, s.site_mask, s.q, s.sigma,
+                      s.epsilon, s.rscreen).eval(s.positions)
+    ref = None
+    # fixed-point sums: the same bits whatever the list holds beyond the cutoff
+    for width in (0.3, 1.5):
+        g = ElecLJ(precision="mixed", neighbor_list_width=width, **cfg).init(s).compute(s.positions, want_fields=True)
+        assert rel_rms(g["f"], o["f"]) < 1e-5
+        assert rel_rms(g["phi"], o["phi"]) < 1e-5
+        assert abs(g["total"] - o["total"]) < 5e-5 * abs(o["total"])
+        if ref is not None:
+            assert np.array_equal(g["f"], ref["f"]) and g["lj"] == ref["lj"]
+        ref = g
