@@ -642,7 +642,7 @@ extern "C" int mmnb_backward(mmnb_handle *h, const double *r, const double *dl_d
     return s;
   double acc[6] = {0, 0, 0, 0, 0, 0};
   for (size_t i = 0; i < n; i++) {
-    const double p[3] = {h->hq[i], h->hsig[i], h->heps[i]};
+    const double p[3] = {h->hpar[i], h->hpar[n + i], h->hpar[2 * n + i]};
     for (int k = 0; k < 6; k++)
       acc[k] += p[k % 3] * g[k * n + i];
   }

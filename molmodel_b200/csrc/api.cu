@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <set>
 #include <string>
 #include <tuple>
@@ -489,7 +490,7 @@ void free_all(mmnb_handle *h)
     h->copy_in = nullptr;
   }
   void *ptrs[] = {h->d_group, h->d_excl_ptr, h->d_excl_idx, h->d_p14_ptr, h->d_p14_idx, h->d_gexcl_ptr,
-                  h->d_gexcl_idx, h->d_mask, h->d_q, h->d_sig, h->d_eps, h->d_rscreen, h->d_cheb_w, h->d_cheb_d, h->d_lj_row, h->d_lj_row_part,
+                  h->d_gexcl_idx, h->d_q, h->d_cheb_w, h->d_cheb_d, h->d_lj_row, h->d_lj_row_part,
                   h->d_vir_part, h->d_vir_row, h->d_vir_mol, h->d_vir_molw, h->d_vir_mass,
                   h->d_stencil, h->d_cell_rank, h->d_cell_of_rank, h->d_cell_of_group, h->d_cell_count,
                   h->d_cell_start, h->d_slot, h->d_sorted, h->d_rank, h->d_anchor, h->d_last, h->d_anchor_sorted, h->d_anchor32, h->d_block_sum,
@@ -752,9 +753,13 @@ static int create_impl(mmnb_handle *h, const mmnb_config *c, int nsite, int ngro
       (s = upload(h, &h->d_p14_idx, h->p14_idx)) || (s = upload(h, &h->d_gexcl_ptr, h->gexcl_ptr)) ||
       (s = upload(h, &h->d_gexcl_idx, h->gexcl_idx)))
     return s;
-  if ((s = dalloc(h, &h->d_mask, nsite)) || (s = dalloc(h, &h->d_q, nsite)) || (s = dalloc(h, &h->d_sig, nsite)) ||
-      (s = dalloc(h, &h->d_eps, nsite)) || (s = dalloc(h, &h->d_rscreen, nsite)))
+  // the site parameters in one block: mmnb_set_params fills it with one copy
+  if ((s = dalloc(h, &h->d_q, 5 * (size_t) nsite)))
     return s;
+  h->d_sig = h->d_q + nsite;
+  h->d_eps = h->d_sig + nsite;
+  h->d_rscreen = h->d_eps + nsite;
+  h->d_mask = reinterpret_cast<int *>(h->d_rscreen + nsite);
   if ((s = dalloc(h, &h->d_cell_of_group, ngroup)) || (s = dalloc(h, &h->d_slot, ngroup)) ||
       (s = dalloc(h, &h->d_sorted, ngroup)) || (s = dalloc(h, &h->d_rank, ngroup)) ||
       (s = dalloc(h, &h->d_anchor, 3 * (size_t) ngroup)) || (s = dalloc(h, &h->d_last, 3 * (size_t) ngroup)) ||
@@ -868,7 +873,6 @@ int mmnb_set_params(mmnb_handle *h, const int *site_mask, const double *q, const
   drop_host_graph(h);
   h->buf_gen++;  // the kernels an evaluation launches may change
   const int n = h->nsite;
-  std::vector<double> rs(n, 0.0);
   h->any_q = h->any_lj = h->has_rscreen = false;
   h->lj_on_anchors_only = true;
   double qsum = 0;
@@ -885,45 +889,64 @@ int mmnb_set_params(mmnb_handle *h, const int *site_mask, const double *q, const
     if (rscreen) {
       if (rscreen[i] < 0)
         return fail(h, MMNB_ERR_ARG, "screening radius must be >= 0");
-      rs[i] = rscreen[i];
       if (rscreen[i] > 0)
         h->has_rscreen = true;
     }
     qsum += q[i];
   }
-  CK(cudaMemcpy(h->d_mask, site_mask, sizeof(int) * n, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(h->d_q, q, sizeof(double) * n, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(h->d_sig, sig, sizeof(double) * n, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(h->d_eps, eps, sizeof(double) * n, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(h->d_rscreen, rs.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
+  // one copy, in order with the work of the handle's stream
+  h->hpar.resize(4 * (size_t) n + (n + 1) / 2);
+  double *par = h->hpar.data();
+  std::copy(q, q + n, par);
+  std::copy(sig, sig + n, par + n);
+  std::copy(eps, eps + n, par + 2 * (size_t) n);
+  if (rscreen)
+    std::copy(rscreen, rscreen + n, par + 3 * (size_t) n);
+  else
+    std::fill(par + 3 * (size_t) n, par + 4 * (size_t) n, 0.0);
+  memcpy(par + 4 * (size_t) n, site_mask, sizeof(int) * n);
+  CK(cudaMemcpyAsync(h->d_q, par, sizeof(double) * 4 * (size_t) n + sizeof(int) * n, cudaMemcpyHostToDevice,
+                     h->stream));
   h->grad_ready = false;
-  h->hq.assign(q, q + n);
-  h->hsig.assign(sig, sig + n);
-  h->heps.assign(eps, eps + n);
   // LJ tail totals over distinct (sigma, epsilon) printed as %12.6g
   // (src/eleclj.cpp:283-308)
   h->cls_sig.clear();
   h->cls_eps.clear();
   h->cls_n.clear();
   h->site_cls.assign(n, -1);
+  // sites with the same bits are of one class: each distinct pair is printed once
+  std::map<std::pair<double, double>, int> seen;
+  int last = -1;
   for (int i = 0; i < n; i++) {
     if (!(site_mask[i] & MMNB_SITE_HAS_LJ))
       continue;
-    char key[128];
-    double sv, ev;
-    snprintf(key, sizeof key, "%12.6g %12.6g", sig[i], eps[i]);
-    sscanf(key, "%lf%lf", &sv, &ev);
-    size_t a = 0;
-    for (; a < h->cls_sig.size(); a++)
-      if (h->cls_sig[a] == sv && h->cls_eps[a] == ev)
-        break;
-    if (a == h->cls_sig.size()) {
-      h->cls_sig.push_back(sv);
-      h->cls_eps.push_back(ev);
-      h->cls_n.push_back(0);
+    int a = -1;
+    if (last >= 0 && sig[i] == sig[last] && eps[i] == eps[last]) {
+      a = h->site_cls[last];
+    } else if (eps[i] == eps[i]) {  // (NaN has no place in an ordered map)
+      const auto it = seen.find(std::make_pair(sig[i], eps[i]));
+      if (it != seen.end())
+        a = it->second;
+    }
+    if (a < 0) {
+      char key[128];
+      double sv, ev;
+      snprintf(key, sizeof key, "%12.6g %12.6g", sig[i], eps[i]);
+      sscanf(key, "%lf%lf", &sv, &ev);
+      a = 0;
+      while (a < (int) h->cls_sig.size() && !(h->cls_sig[a] == sv && h->cls_eps[a] == ev))
+        a++;
+      if (a == (int) h->cls_sig.size()) {
+        h->cls_sig.push_back(sv);
+        h->cls_eps.push_back(ev);
+        h->cls_n.push_back(0);
+      }
+      if (eps[i] == eps[i])
+        seen[std::make_pair(sig[i], eps[i])] = a;
     }
     h->cls_n[a]++;
-    h->site_cls[i] = (int) a;
+    h->site_cls[i] = a;
+    last = i;
   }
   h->totA = h->totB = 0;
   for (size_t a = 0; a < h->cls_sig.size(); a++)
@@ -1416,11 +1439,10 @@ int mmnb_scale(mmnb_handle *h, double s)
   if ((st = setup_cells(h)))
     return st;
   // q sum for the neutralising term
-  std::vector<double> q(h->nsite);
-  CK(cudaMemcpy(q.data(), h->d_q, sizeof(double) * h->nsite, cudaMemcpyDeviceToHost));
   double qsum = 0;
-  for (double v : q)
-    qsum += v;
+  if (h->params_set)
+    for (int i = 0; i < h->nsite; i++)
+      qsum += h->hpar[i];
   update_energy_constants(h, qsum);
   CK(cudaStreamSynchronize(h->stream));
   return MMNB_OK;

@@ -229,7 +229,7 @@ struct mmnb_handle {
   // host copies of the site parameters, and the LJ classes of the tail:
   // distinct (sigma, epsilon) as printed with %12.6g, their site counts, and
   // each site's class (-1 without LJ)
-  std::vector<double> hq, hsig, heps;
+  std::vector<double> hpar;          // as copied to the device: q, sigma, epsilon, r_screen, masks
   std::vector<double> cls_sig, cls_eps;
   std::vector<long> cls_n;
   std::vector<int> site_cls;
