@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(kGradWarps * 32) k_grad_pair(GradArgs a)
 }
 
 // exclusion corrections and 1-4 pairs, one thread per site over its own
-// partners (the forward's k_exclusions_fp64 terms)
+// partners (the forward's terms in k_sites)
 __global__ void __launch_bounds__(kGradThreads) k_grad_excl(GradArgs a)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

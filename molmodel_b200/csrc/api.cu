@@ -262,7 +262,8 @@ int setup_cells(mmnb_handle *h)
   }
   if ((s = upload(h, &h->d_cell_rank, rank)) || (s = upload(h, &h->d_cell_of_rank, of_rank)))
     return s;
-  if ((s = dalloc(h, &h->d_cell_count, h->ncell3)) || (s = dalloc(h, &h->d_cell_start, h->ncell3 + 1)))
+  if ((s = dalloc(h, &h->d_cell_count, h->ncell3)) || (s = dalloc(h, &h->d_cell_start, h->ncell3 + 1)) ||
+      (s = dalloc(h, &h->d_cell_head, h->ncell3)))
     return s;
   h->first = true;
   return MMNB_OK;
@@ -490,16 +491,16 @@ void free_all(mmnb_handle *h)
     h->copy_in = nullptr;
   }
   void *ptrs[] = {h->d_group, h->d_excl_ptr, h->d_excl_idx, h->d_p14_ptr, h->d_p14_idx, h->d_gexcl_ptr,
-                  h->d_gexcl_idx, h->d_q, h->d_cheb_w, h->d_cheb_d, h->d_lj_row, h->d_lj_row_part,
-                  h->d_vir_part, h->d_vir_row, h->d_vir_mol, h->d_vir_molw, h->d_vir_mass,
+                  h->d_gexcl_idx, h->d_q, h->d_cheb_w, h->d_cheb_d, h->d_lj_row,
+                  h->d_vir_row, h->d_vir_mol, h->d_vir_molw, h->d_vir_mass,
                   h->d_stencil, h->d_cell_rank, h->d_cell_of_rank, h->d_cell_of_group, h->d_cell_count,
-                  h->d_cell_start, h->d_slot, h->d_sorted, h->d_rank, h->d_anchor, h->d_last, h->d_anchor_sorted, h->d_anchor32, h->d_block_sum,
+                  h->d_cell_start, h->d_cell_head, h->d_slot, h->d_sorted, h->d_rank, h->d_anchor, h->d_last, h->d_anchor_sorted, h->d_anchor32,
                   h->d_top2, h->d_nbr, h->d_nbr_count, h->d_pnbr, h->d_pcount, h->d_plast, h->d_flags, h->d_sr,
                   h->d_sp, h->d_sanchor, h->d_site_of_slot,
-                  h->d_phi, h->d_evec, h->d_ljf, h->d_lj_part, h->d_elec_part, h->d_energy, h->d_r, h->d_f,
+                  h->d_phi, h->d_evec, h->d_ljf, h->d_site_part, h->d_energy, h->d_r, h->d_f,
                   h->d_mesh, h->d_meshk, h->d_green, h->d_kvec, h->d_egrid, h->d_egridk, h->d_mesh32,
                   h->d_meshk32, h->d_green32, h->d_egrid32, h->d_egridk32, h->d_mesh_fx,
-                  h->mx.site, h->mx.par, h->mx.anchor, h->mx.anc32, h->mx.acc, h->mx.acck, h->d_wsum,
+                  h->mx.site, h->mx.par, h->mx.anchor, h->mx.anc32, h->mx.acc, h->d_wsum,
                   h->d_bwd, h->d_esp, h->d_gmesh, h->d_gmeshk, h->d_chi_part};
   for (void *p : ptrs)
     if (p)
@@ -766,15 +767,6 @@ static int create_impl(mmnb_handle *h, const mmnb_config *c, int nsite, int ngro
       (s = dalloc(h, &h->d_anchor_sorted, 3 * (size_t) ngroup)) || (s = dalloc(h, &h->d_anchor32, ngroup)) ||
       (s = dalloc(h, &h->d_nbr_count, ngroup)) || (s = dalloc(h, &h->d_flags, kFlagCount)))
     return s;
-  {
-    // one word per block of the cooperative rebuild (at most 2048 threads of
-    // 256-thread blocks resident per SM)
-    int nsm = 0;
-    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->dev));
-    h->block_sum_cap = 8 * nsm;
-    if ((s = dalloc(h, &h->d_block_sum, (size_t) h->block_sum_cap)))
-      return s;
-  }
   CK(cudaMemset(h->d_last, 0, sizeof(double) * 3 * ngroup));
   CK(cudaMemset(h->d_flags, 0, sizeof(int) * kFlagCount));
   CK(cudaMallocHost((void **) &h->h_flags, sizeof(int) * kFlagCount));
@@ -787,25 +779,17 @@ static int create_impl(mmnb_handle *h, const mmnb_config *c, int nsite, int ngro
       (s = dalloc(h, &h->d_sanchor, ngroup)) ||
       (s = dalloc(h, &h->d_site_of_slot, nslot)))
     return s;
-  h->elec_blocks = div_up(nsite, 256);
-  h->lj_pair_blocks = pair_blocks(h);
-  h->lj_excl_blocks = excl_blocks(h);
-  const size_t nlj = (size_t) h->lj_pair_blocks + h->lj_excl_blocks;
   if ((s = dalloc(h, &h->d_phi, nsite)) || (s = dalloc(h, &h->d_evec, 3 * (size_t) nsite)) ||
-      (s = dalloc(h, &h->d_ljf, 3 * (size_t) nsite)) || (s = dalloc(h, &h->d_lj_part, nlj)) ||
-      (s = dalloc(h, &h->d_lj_row, ngroup)) || (s = dalloc(h, &h->d_vir_part, nlj)) ||
-      (s = dalloc(h, &h->d_vir_row, ngroup)) ||
-      (s = dalloc(h, &h->d_elec_part, h->elec_blocks)) || (s = dalloc(h, &h->d_lj_row_part, h->elec_blocks)) || (s = dalloc(h, &h->d_energy, 16)) ||
-      (s = dalloc(h, &h->d_r, 3 * (size_t) nsite)) || (s = dalloc(h, &h->d_f, 3 * (size_t) nsite)) ||
-      (s = dalloc(h, &h->d_wsum, 8)))
+      (s = dalloc(h, &h->d_ljf, 3 * (size_t) nsite)) || (s = dalloc(h, &h->d_lj_row, ngroup)) ||
+      (s = dalloc(h, &h->d_vir_row, ngroup)) || (s = dalloc(h, &h->d_site_part, 4 * (size_t) site_blocks(h))) ||
+      (s = dalloc(h, &h->d_energy, 16)) || (s = dalloc(h, &h->d_r, 3 * (size_t) nsite)) ||
+      (s = dalloc(h, &h->d_f, 3 * (size_t) nsite)) || (s = dalloc(h, &h->d_wsum, 8)))
     return s;
-  CK(cudaMemset(h->d_lj_part, 0, sizeof(double) * nlj));
   CK(cudaMemset(h->d_wsum, 0, sizeof(unsigned long long) * 8));
   if (c->precision == MMNB_MIXED) {
     if ((s = dalloc(h, &h->mx.site, nslot)) || (s = dalloc(h, &h->mx.par, nslot)) ||
         (s = dalloc(h, &h->mx.anchor, ngroup)) || (s = dalloc(h, &h->mx.anc32, ngroup)) ||
-        (s = dalloc(h, &h->mx.acc, (size_t) nsite * kAccStride)) ||
-        (s = dalloc(h, &h->mx.acck, (size_t) nsite * 4)))
+        (s = dalloc(h, &h->mx.acc, (size_t) nsite * kAccStride)))
       return s;
     CK(cudaMemset(h->mx.acc, 0, sizeof(long long) * nsite * kAccStride));
   }
@@ -1004,34 +988,18 @@ int mmnb_compute_device(mmnb_handle *h, const double *d_r, double *d_f, double *
   timing_mark(h, "start");
   // P3M charge assignment and FFTs depend only on the positions: they run on
   // the side stream while the list and pair kernels run here, and are joined
-  // back before k_finalize (FP64 form: before the interpolation, which adds
-  // to what the pair kernels wrote).  With stage timing on, the join follows
+  // back before k_sites, which interpolates.  With stage timing on, the join follows
   // at once so the marks stay serial.
   const bool p3m = h->any_q && h->cfg.include_kspace && h->p3m;
   // the side stream pays off when the pair kernels leave room beside them;
   // mmnb_autotune may put the mesh work in line instead (tune.p3m_side = 0)
   const bool side = p3m && h->tune.p3m_side;
-  // the mixed form's FP64 site arrays (written by the exclusion corrections)
-  // do not meet the pair kernels either: they go to the side stream too
-  const bool excl_side = side && mixed && h->cfg.include_rspace;
-  auto zero_site_arrays = [&]() -> cudaError_t {
-    cudaError_t e;
-    if ((e = cudaMemsetAsync(h->d_phi, 0, sizeof(double) * h->nsite, h->stream)) != cudaSuccess ||
-        (e = cudaMemsetAsync(h->d_evec, 0, sizeof(double) * 3 * h->nsite, h->stream)) != cudaSuccess)
-      return e;
-    return cudaMemsetAsync(h->d_ljf, 0, sizeof(double) * 3 * h->nsite, h->stream);
-  };
-  // the mixed form's interpolation writes words of its own (k_gather_mixed),
-  // so it joins the mesh work; the FP64 interpolation adds into the site
-  // arrays the pair kernels write and waits for them
-  const int mesh_stages = mixed ? 3 : 1;
   if (side) {
     cudaStream_t main = h->stream;
     CK(cudaEventRecord(h->ev_fork, main));
     CK(cudaStreamWaitEvent(h->side, h->ev_fork, 0));
     h->stream = h->side;
     cudaError_t e = cudaSuccess;
-    int stages = mesh_stages;
     if (h->in_chunks) {
       // the host call's positions arrive in pieces: each piece's charges are
       // assigned as it lands (mixed form), the rest follows the last piece
@@ -1042,15 +1010,9 @@ int mmnb_compute_device(mmnb_handle *h, const double *d_r, double *d_f, double *
         if (e == cudaSuccess && mixed)
           e = launch_spread_mixed_range(h, d_r, lo, hi);
       }
-      if (mixed)
-        stages |= 4;
-    }
-    if (excl_side && e == cudaSuccess) {
-      e = launch_exclusions(h, d_r);
-      timing_mark(h, "rspace_excl");
     }
     if (e == cudaSuccess)
-      e = mixed ? launch_p3m_mixed(h, d_r, stages) : launch_p3m_fp64(h, d_r, stages);
+      e = mixed ? launch_p3m_mixed(h, d_r, h->in_chunks) : launch_p3m_fp64(h, d_r);
     h->stream = main;
     CK(e);
     CK(cudaEventRecord(h->ev_join, h->side));
@@ -1077,15 +1039,10 @@ int mmnb_compute_device(mmnb_handle *h, const double *d_r, double *d_f, double *
   if (h->in_chunks)
     CK(cudaStreamWaitEvent(h->stream, h->ev_in[mmnb_handle::kInChunks - 1], cudaEventWaitExternal));
   if (p3m && !side)
-    CK(mixed ? launch_p3m_mixed(h, d_r, mesh_stages) : launch_p3m_fp64(h, d_r, mesh_stages));
+    CK(mixed ? launch_p3m_mixed(h, d_r, false) : launch_p3m_fp64(h, d_r));
   CK(launch_list_check(h, d_r, h->force_rebuild_next));
-  CK(launch_list_rebuild(h));
+  CK(launch_list_cells(h));
   timing_mark(h, "nbrlist");
-  // FP64 site arrays collect the terms the fixed-point sums do not hold; their
-  // first writer (FP64 pair kernels, or the mixed form's exclusion
-  // corrections) assigns them, so they need clearing only without real space
-  if (!h->cfg.include_rspace)
-    CK(zero_site_arrays());
   // FP64 rigid water: its own kernel (any request, site fields included)
   const bool water64 = !mixed && h->water && h->cfg.include_rspace;
   if (mixed)
@@ -1112,31 +1069,25 @@ int mmnb_compute_device(mmnb_handle *h, const double *d_r, double *d_f, double *
       h->used_rows64 = true;
     }
     timing_mark(h, "rspace_pair");
-    if (!excl_side) {
-      CK(launch_exclusions(h, d_r));
-      timing_mark(h, "rspace_excl");
-    }
-  } else {
-    CK(cudaMemsetAsync(h->d_lj_part, 0, sizeof(double) * (h->lj_pair_blocks + h->lj_excl_blocks), h->stream));
-    if (mixed)
-      CK(cudaMemsetAsync(h->mx.acc, 0, sizeof(long long) * h->nsite * kAccStride, h->stream));
+  } else if (mixed) {
+    CK(cudaMemsetAsync(h->mx.acc, 0, sizeof(long long) * h->nsite * kAccStride, h->stream));
   }
+  h->used_ksum = ksum;
   if (p3m) {
     if (side && !h->timing.on)
       CK(cudaStreamWaitEvent(h->stream, h->ev_join, 0));
-    if (!mixed)
-      CK(launch_p3m_fp64(h, d_r, 2));
-    timing_mark(h, "kspace");
   } else if (ksum) {
     if (!h->tune.p3m_side)
       CK(launch_ewald_structure(h, h->ew, d_r, nullptr));
     else if (!h->timing.on)
       CK(cudaStreamWaitEvent(h->stream, h->ev_join, 0));
-    CK(launch_ewald_sum(h, h->ew, h->nsite, d_r, 0.0, h->d_phi, h->d_evec));
+    // added to what the FP64 pair kernels wrote; otherwise the site arrays' first term
+    const bool add = !mixed && h->cfg.include_rspace;
+    CK(launch_ewald_sum(h, h->ew, h->nsite, d_r, 0.0, h->d_phi, h->d_evec, add));
     timing_mark(h, "kspace");
   }
-  CK(launch_finalize(h, d_f, energy));
-  timing_mark(h, "finalize");
+  CK(launch_sites(h, d_r, d_f, energy));
+  timing_mark(h, "sites");
   h->first = false;
   h->force_rebuild_next = 0;
   h->evals++;
@@ -1224,9 +1175,9 @@ static int compute_host(mmnb_handle *h, const double *r, double *f, double *u, m
   volatile unsigned long long *ready =
       reinterpret_cast<volatile unsigned long long *>(h->h_status) + mmnb_handle::kStatusReady;
   for (int attempt = 0; attempt < 2; attempt++) {
-    *ready = 0ull;  // k_finalize sets it once this evaluation's status is in place
+    *ready = 0ull;  // k_sites sets it once this evaluation's status is in place
     // after the first call, a plain evaluation replays the handle's own graph
-    // (zeroing, list check/rebuild, pair and mesh kernels, finalize)
+    // (zeroing, list check/rebuild, pair and mesh kernels, sites)
     const bool graph =
         !h->first && !(phi || evec || keep) && !h->timing.on && !h->force_rebuild_next && !h->want_virial;
     if (graph) {
@@ -1256,12 +1207,12 @@ static int compute_host(mmnb_handle *h, const double *r, double *f, double *u, m
       h->capturing = true;
       h->in_chunks = true;
       const long ev = h->evals, ln = h->launches;
-      cudaError_t ce = cudaMemsetAsync(h->d_f, 0, sizeof(double) * n3, h->stream);
-      if (ce == cudaSuccess)
-        ce = cudaMemsetAsync(h->d_flags + kFlagOverflow, 0, sizeof(int), h->stream);
+      const cudaError_t ce = cudaMemsetAsync(h->d_flags + kFlagOverflow, 0, sizeof(int), h->stream);
       h->want_status = true;
+      h->assign_forces = true;
       const int s = ce == cudaSuccess ? mmnb_compute_device(h, h->d_r, h->d_f, h->d_energy) : MMNB_ERR_CUDA;
       h->want_status = false;
+      h->assign_forces = false;
       h->capturing = false;
       h->in_chunks = false;
       cudaGraph_t g = nullptr;
@@ -1284,11 +1235,12 @@ static int compute_host(mmnb_handle *h, const double *r, double *f, double *u, m
       h->evals++;
       h->launches += h->host_launch_per_eval;
     } else {
-      CK(cudaMemsetAsync(h->d_f, 0, sizeof(double) * n3, h->stream));
       CK(cudaMemsetAsync(h->d_flags + kFlagOverflow, 0, sizeof(int), h->stream));
       h->want_fields = phi || evec || keep;
       h->want_status = true;
+      h->assign_forces = true;
       const int s = mmnb_compute_device(h, h->d_r, h->d_f, h->d_energy);
+      h->assign_forces = false;
       h->want_status = false;
       h->want_fields = false;
       if (s)

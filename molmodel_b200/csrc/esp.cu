@@ -428,7 +428,7 @@ extern "C" int mmnb_phi_at_points(mmnb_handle *h, const double *r, int npoint, c
   if (e == cudaSuccess && (nk > 0 || neutral != 0)) {
     EwaldSum none;
     none.made = true;
-    e = launch_ewald_sum(h, nk > 0 ? h->ew : none, npoint, d_pts, neutral, d_phi, nullptr);
+    e = launch_ewald_sum(h, nk > 0 ? h->ew : none, npoint, d_pts, neutral, d_phi, nullptr, true);
   }
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(phi, d_phi, npoint * sizeof(double), cudaMemcpyDeviceToHost, h->stream);

@@ -162,12 +162,12 @@ __global__ void __launch_bounds__(32 * kEwSlices) k_ewald_reduce(EwaldArgs a, in
   }
 }
 
-// phi (and with FIELD the field) of a lane's site or point, added to phi / evec
+// phi (and with FIELD the field) of a lane's site or point
 // STAGED: S(k) and the rows come from shared memory (each warp's walk over them is a
 // chain of dependent reads)
 template <bool FIELD, bool STAGED>
-__global__ void __launch_bounds__(32 * kEwWarps) k_ewald_sum(EwaldArgs a, double neutral, double *__restrict__ phi,
-                                                             double *__restrict__ evec)
+__global__ void __launch_bounds__(32 * kEwWarps) k_ewald_sum(EwaldArgs a, double neutral, bool add,
+                                                             double *__restrict__ phi, double *__restrict__ evec)
 {
   extern __shared__ __align__(16) double2 tab[];  // [axis][n][site], then S(k) and the rows
   __shared__ double sum[kEwWarps][FIELD ? 4 : 1][32];
@@ -250,9 +250,9 @@ __global__ void __launch_bounds__(32 * kEwWarps) k_ewald_sum(EwaldArgs a, double
       v += sum[j][w][lane];
     const size_t i = i0 + lane;
     if (w == 0)
-      phi[i] = (phi[i] + v) + neutral;
+      phi[i] = ((add ? phi[i] : 0.0) + v) + neutral;
     else
-      evec[3 * i + w - 1] += v * a.rec[w - 1];
+      evec[3 * i + w - 1] = (add ? evec[3 * i + w - 1] : 0.0) + v * a.rec[w - 1];
   }
 }
 
@@ -380,7 +380,7 @@ cudaError_t launch_ewald_structure(mmnb_handle *h, const EwaldSum &e, const doub
 }
 
 cudaError_t launch_ewald_sum(mmnb_handle *h, const EwaldSum &e, int n, const double *d_pts, double neutral,
-                             double *d_phi, double *d_evec)
+                             double *d_phi, double *d_evec, bool add)
 {
   EwaldArgs a = ewald_args(h, e);
   a.n = n;
@@ -398,7 +398,7 @@ cudaError_t launch_ewald_sum(mmnb_handle *h, const EwaldSum &e, int n, const dou
     if (s != cudaSuccess)
       return s;
   }
-  k<<<div_up(n, a.tile), 32 * kEwWarps, smem, h->stream>>>(a, neutral, d_phi, d_evec);
+  k<<<div_up(n, a.tile), 32 * kEwWarps, smem, h->stream>>>(a, neutral, add, d_phi, d_evec);
   h->launches += 1;
   return cudaGetLastError();
 }
@@ -413,7 +413,7 @@ cudaError_t launch_kspace_dipole(mmnb_handle *h, const double *d_r, const double
   if (h->ew.nk == 0)
     return cudaSuccess;
   const cudaError_t e = launch_ewald_structure(h, h->ew, d_r, d_g);
-  return e != cudaSuccess ? e : launch_ewald_sum(h, h->ew, h->nsite, d_r, 0.0, d_psi, nullptr);
+  return e != cudaSuccess ? e : launch_ewald_sum(h, h->ew, h->nsite, d_r, 0.0, d_psi, nullptr, true);
 }
 
 }  // namespace mmnb

@@ -416,14 +416,13 @@ static int md_record(mmnb_md *md, double *log)
   const MdArgs a = md_args(md, log);
   const int n = md->rigid ? md->nmol : md->nsite;
   k_md_drift<<<div_up(n, 128), 128, 0, h->stream>>>(a);
-  cudaError_t e = cudaMemsetAsync(md->d_f, 0, 3 * (size_t) md->nsite * sizeof(double), h->stream);
-  if (e != cudaSuccess)
-    return md_fail(md, MMNB_ERR_CUDA, cudaGetErrorString(e));
+  h->assign_forces = true;
   const int s = mmnb_compute_device(h, md->d_r, md->d_f, md->d_energy);
+  h->assign_forces = false;
   if (s)
     return md_fail(md, s, mmnb_last_error(h));
   k_md_kick<<<md->ke_blocks, kMdThreads, 0, h->stream>>>(a, 1);
-  e = cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess)
     return md_fail(md, MMNB_ERR_CUDA, cudaGetErrorString(e));
   return MMNB_OK;

@@ -70,7 +70,6 @@ struct MixedBufs {
   float4 *anc32 = nullptr;       // rigid-water kernel, sorted groups: the anchor's offset from the corner
                                  // of its list cell (FP32) and the cell's coordinates (10 bits each, in w)
   long long *acc = nullptr;      // per site (original order), kAccStride fixed-point values
-  long long *acck = nullptr;     // per site (original order): P3M interpolation phi, Ex, Ey, Ez
 };
 
 // Wave vectors and sums of the ordinary Ewald reciprocal space (kspace.cu)
@@ -159,7 +158,8 @@ struct mmnb_handle {
   int *d_cell_of_group = nullptr;    // per group, reference numbering
   int *d_cell_count = nullptr;       // per rank
   int *d_cell_start = nullptr;       // per rank, ncell3+1
-  int *d_slot = nullptr;             // per group, slot inside its cell
+  int *d_cell_head = nullptr;        // per rank, the cell's last group to arrive
+  int *d_slot = nullptr;             // per group, the group that arrived in its cell before
   int *d_sorted = nullptr;           // sorted position -> group
   int *d_rank = nullptr;             // group -> sorted position
   double *d_anchor = nullptr;        // 3*ngroup current anchors (original order)
@@ -168,9 +168,6 @@ struct mmnb_handle {
   float4 *d_anchor32 = nullptr;      // the same, wrapped into the box, FP32 (list pre-test)
   double *d_top2 = nullptr;          // per-block top-2 displacements
   int top2_blocks = 0;
-  int rebuild_grid = 0;              // blocks of the cooperative rebuild launch (0: not sized yet)
-  int *d_block_sum = nullptr;        // per rebuild block: its segment's cell count
-  int block_sum_cap = 0;
   int rowcap = 0;
   int *d_nbr = nullptr;              // ngroup * rowcap, sorted positions
   int *d_nbr_count = nullptr;        // ngroup
@@ -199,18 +196,16 @@ struct mmnb_handle {
 
   // outputs (original order)
   double *d_phi = nullptr, *d_evec = nullptr, *d_ljf = nullptr;
-  double *d_lj_part = nullptr;       // LJ energy partials: pair-kernel blocks, then exclusion blocks
-  double *d_lj_row = nullptr;        // FP64 water kernel: LJ energy of each row (sorted order)
-  double *d_lj_row_part = nullptr;   // finalize: per block, its slice of d_lj_row
-  // mmnb_virial: the pair kernels' virial term (per block: pair-kernel blocks,
-  // then exclusion blocks; per row: FP64 water kernel), molecule ranges,
+  double *d_lj_row = nullptr;        // FP64 pair kernels: LJ energy of each row (sorted order)
+  double *d_site_part = nullptr;     // site kernel: per block, its four partial sums
+  // mmnb_virial: the FP64 pair kernels' virial term per row, molecule ranges,
   // masses and per-molecule sums (allocated on first use)
-  double *d_vir_part = nullptr, *d_vir_row = nullptr;
+  double *d_vir_row = nullptr;
   int *d_vir_mol = nullptr;
   double *d_vir_molw = nullptr, *d_vir_mass = nullptr;
   int vir_mol_cap = 0;
   // [0], [1]: fixed-point Coulomb (rigid water) and LJ pair energies of the mixed pair kernels;
-  // [2]: block counter of the finalize kernel's last-block reduction;
+  // [2]: block counter of the site kernel's last-block reduction;
   // [3]: row counter of the FP64 pair kernels; [4]: the mixed pair kernels'
   // fixed-point virial term
   unsigned long long *d_wsum = nullptr;
@@ -233,10 +228,7 @@ struct mmnb_handle {
   std::vector<double> cls_sig, cls_eps;
   std::vector<long> cls_n;
   std::vector<int> site_cls;
-  int lj_pair_blocks = 0, lj_excl_blocks = 0;
-  double *d_elec_part = nullptr;     // per block
-  int elec_blocks = 0;
-  double *d_energy = nullptr;        // 4 doubles
+  double *d_energy = nullptr;        // 4 doubles; [8]: the 1-4 pairs' virial term
   // host path staging
   double *d_r = nullptr, *d_f = nullptr;
   double *h_r = nullptr, *h_f = nullptr, *h_out = nullptr;  // pinned
@@ -293,7 +285,7 @@ struct mmnb_handle {
   cudaEvent_t ev_in[kInChunks] = {};
   cudaEvent_t ev_free = nullptr;  // the handle's stream has let go of d_r
   bool in_chunks = false;         // set while that graph is captured
-  // the host call's status block in mapped pinned memory: k_finalize writes
+  // the host call's status block in mapped pinned memory: k_sites writes
   // the energies [0, 4), the flags (ints, from double 4 on) and then, after a
   // system-wide fence, the ready word; the host spins on that word instead of
   // copying the block back after the evaluation
@@ -301,6 +293,8 @@ struct mmnb_handle {
   static constexpr int kStatusReady = 15;  // double slot of the ready word
   double *h_status = nullptr;
   double *d_status = nullptr;  // its device alias
+  bool assign_forces = false;  // this evaluation writes d_f instead of adding to it
+  bool used_ksum = false;      // the last evaluation ran the k-sum
   bool want_status = false;    // set while the host call records its evaluation: no
                                // other evaluation writes the block
   bool capturing = false;
@@ -313,9 +307,10 @@ namespace mmnb {
 void drop_host_graph(mmnb_handle *h);
 // LJ tail correction (src/eleclj.cpp:1247-1266) for totals A and B; linear in both
 double lj_tail_ab(const mmnb_handle *h, double A, double B);
-// anchors, rebuild decision; then the rebuild (a no-op launch when not due)
+// anchors, rebuild decision; then the cells and sorted order of a rebuild (a no-op
+// launch when not due); the rows are built by the site-sorting kernels (nbrlist.cuh)
 cudaError_t launch_list_check(mmnb_handle *h, const double *d_r, int force);
-cudaError_t launch_list_rebuild(mmnb_handle *h);
+cudaError_t launch_list_cells(mmnb_handle *h);
 cudaError_t launch_sort_sites(mmnb_handle *h, const double *d_r);
 cudaError_t launch_rspace_fp64(mmnb_handle *h);
 cudaError_t launch_prep_mixed(mmnb_handle *h, const double *d_r);
@@ -323,10 +318,9 @@ cudaError_t launch_rspace_mixed(mmnb_handle *h);
 cudaError_t launch_rspace_water(mmnb_handle *h);
 cudaError_t launch_sort_water64(mmnb_handle *h, const double *d_r);
 cudaError_t launch_rspace_water64(mmnb_handle *h);
-cudaError_t launch_exclusions(mmnb_handle *h, const double *d_r);
 cudaError_t launch_p3m_green(mmnb_handle *h, double eta, double *chi);
-// stage bit 1: spread + FFT round trip, bit 2: gather
-cudaError_t launch_p3m_fp64(mmnb_handle *h, const double *d_r, int stage);
+// charge assignment and FFT round trip
+cudaError_t launch_p3m_fp64(mmnb_handle *h, const double *d_r);
 // FP64 meshes and plans of the adjoint's dipole solve: spread/spreadk hold one
 // mesh (three with ik differentiation); solvek/solve the summed ik spectrum
 // and its transform (ik only; otherwise the solve happens in place)
@@ -340,13 +334,13 @@ cudaError_t launch_p3m_dipole_fp64(mmnb_handle *h, const double *d_r, const doub
                                    double *d_psi);
 // d_psi += reciprocal-sum potential of the dipoles q_j g_j
 cudaError_t launch_kspace_dipole(mmnb_handle *h, const double *d_r, const double *d_g, double *d_psi);
-cudaError_t launch_p3m_mixed(mmnb_handle *h, const double *d_r, int stage);
+// (assigned: the charges are on the mesh already, launch_spread_mixed_range's)
+cudaError_t launch_p3m_mixed(mmnb_handle *h, const double *d_r, bool assigned);
 // write back and drop [p, p + bytes) from the host cores' caches (hostmem.cpp)
 void evict_host_lines(const void *p, size_t bytes);
 
-// the mixed charge assignment of sites [lo, hi) alone; stage bit 4 of
-// launch_p3m_mixed then skips it (the mesh words are integer sums, so the
-// pieces give the mesh of one launch over all sites, bit for bit)
+// the mixed charge assignment of sites [lo, hi) alone (the mesh words are integer
+// sums, so the pieces give the mesh of one launch over all sites, bit for bit)
 cudaError_t launch_spread_mixed_range(mmnb_handle *h, const double *d_r, int lo, int hi);
 cudaError_t launch_green32(mmnb_handle *h);
 // wave vectors of the handle's kspace_cutoff, eta and box (drops what e held)
@@ -354,17 +348,16 @@ cudaError_t ewald_make(mmnb_handle *h, EwaldSum &e);
 void ewald_free(EwaldSum &e);
 // S(k) of the sites at d_r (with d_g: of the dipoles q g) into e.sk
 cudaError_t launch_ewald_structure(mmnb_handle *h, const EwaldSum &e, const double *d_r, const double *d_g);
-// d_phi += potential of e.sk at the n points, + neutral; d_evec (or null) += the field
+// d_phi = (add: +=) potential of e.sk at the n points, + neutral; d_evec (or null) the field
 cudaError_t launch_ewald_sum(mmnb_handle *h, const EwaldSum &e, int n, const double *d_pts, double neutral,
-                             double *d_phi, double *d_evec);
-cudaError_t launch_finalize(mmnb_handle *h, double *d_f, double *d_energy);
-cudaError_t launch_energy(mmnb_handle *h, double *d_energy);
+                             double *d_phi, double *d_evec, bool add);
+// interpolation, exclusions, self terms, forces and energies
+cudaError_t launch_sites(mmnb_handle *h, const double *d_r, double *d_f, double *d_energy);
+int site_blocks(const mmnb_handle *h);  // at most this many blocks
 
 // helpers shared by the .cu files
 void timing_mark(mmnb_handle *h, const char *name);
 int set_global_error(int code, const std::string &msg);  // read back by mmnb_last_error(NULL)
-int pair_blocks(const mmnb_handle *h);
-int excl_blocks(const mmnb_handle *h);
 
 #ifdef __CUDACC__
 // binary search of key in CSR row `row` (sorted)
@@ -397,15 +390,24 @@ static __constant__ double kErfSeries[16] = {
 // operations here, several hundred for erfc and exp (rigid-water FP64 kernel 259 ->
 // 226 us on 32,768 waters).
 constexpr double kErfSeriesMax = 0.85;
-__device__ __forceinline__ void ewald_short(double eta2, double two_eta_rsqrtpi, double r2, double &b0, double &b1)
+
+// p = sqrt(pi) erf(x) / (2 x) and d = dp/dy at y = x^2
+__device__ __forceinline__ void erf_series(double y, double &p, double &d)
 {
-  const double y = eta2 * r2, rinv = rsqrt(r2);
-  double p = kErfSeries[15], d = 0;
+  p = kErfSeries[15];
+  d = 0;
 #pragma unroll
   for (int n = 14; n >= 0; n--) {
     d = fma(d, y, p);
     p = fma(p, y, kErfSeries[n]);
   }
+}
+
+__device__ __forceinline__ void ewald_short(double eta2, double two_eta_rsqrtpi, double r2, double &b0, double &b1)
+{
+  const double rinv = rsqrt(r2);
+  double p, d;
+  erf_series(eta2 * r2, p, d);
   b0 = fma(-two_eta_rsqrtpi, p, rinv);
   b1 = fma(2 * two_eta_rsqrtpi * eta2, d, rinv * rinv * rinv);
 }

@@ -47,7 +47,7 @@
 // Rigid water has its own kernel (rspace_water64.cu), which is faster there (44
 // against 68 us on 4,096 waters, 191 against 392 us on 32,768).
 
-#include "mmnb_internal.cuh"
+#include "nbrlist.cuh"
 
 #include <algorithm>
 
@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(32 * kP64Warps, 1) k_pair_fp64(PairArgs a)
 // charge) and (sigma, sqrt(epsilon), r_screen, -), and per group the anchor with
 // its first site (high word) and number of sites, charged sites and LJ sites (a
 // byte each of the low word: bit k for site k).  Clears the row counter.
-__global__ void k_sort_sites(const double *__restrict__ r, const double *__restrict__ q,
+__device__ __forceinline__ void sort_sites(const double *__restrict__ r, const double *__restrict__ q,
                              const double *__restrict__ sig, const double *__restrict__ eps,
                              const double *__restrict__ rscreen, const int *__restrict__ mask,
                              const int *__restrict__ sorted, const int *__restrict__ group, int ngroup, int G,
@@ -506,152 +506,26 @@ __global__ void k_sort_sites(const double *__restrict__ r, const double *__restr
   }
 }
 
-// Per-site exclusion correction and 1-4 terms: each thread owns one site and
-// adds the partner terms that act on it (src/rspace.c:219-242, 492-557).
-constexpr int kExclThreads = 256;
-
-struct ExclArgs {
-  int nsite;
-  Box box;
-  double eta, e14, l14;
-  int scale_e14, scale_l14, geometric, do14;
-  int assign;  // write the site arrays (first writer of the evaluation) instead of adding
-  const double *r, *q, *sig, *eps, *rscreen;
-  const int *mask, *excl_ptr, *excl_idx, *p14_ptr, *p14_idx;
-  double *phi, *evec, *ljf;
-  double *lj14_part;
-  double *vir14_part;  // per block: the 1-4 LJ force scalars times r^2 / 2 (mmnb_virial), or null
-};
-
-__global__ void __launch_bounds__(kExclThreads) k_exclusions_fp64(ExclArgs a)
+__global__ void __launch_bounds__(32 * kRowWarps)
+k_sort_sites(const double *__restrict__ r, const double *__restrict__ q, const double *__restrict__ sig,
+             const double *__restrict__ eps, const double *__restrict__ rscreen, const int *__restrict__ mask,
+             const int *__restrict__ sorted, const int *__restrict__ group, int ngroup, int G,
+             double4 *__restrict__ sr, double4 *__restrict__ sp, double4 *__restrict__ anchor,
+             unsigned long long *__restrict__ counter, int *__restrict__ flags, RebuildArgs rows)
 {
-  __shared__ double sl[kExclThreads], sv[kExclThreads];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  double elj = 0, vir = 0;
-  if (i < a.nsite) {
-    const int mi = a.mask[i];
-    double phi = 0, ex = 0, ey = 0, ez = 0, lx = 0, ly = 0, lz = 0;
-    const double xi = a.r[3 * i], yi = a.r[3 * i + 1], zi = a.r[3 * i + 2];
-    if (mi & MMNB_SITE_HAS_Q) {
-      for (int n = a.excl_ptr[i]; n < a.excl_ptr[i + 1]; n++) {
-        const int j = a.excl_idx[n];
-        if (!(a.mask[j] & MMNB_SITE_HAS_Q))
-          continue;
-        double x = xi - a.r[3 * j], y = yi - a.r[3 * j + 1], z = zi - a.r[3 * j + 2];
-        min_image_ref(a.box, x, y, z);
-        const double r2 = x * x + y * y + z * z;
-        const double rm = sqrt(r2);
-        const double er = a.eta * rm;
-        const double e = exp(-(er * er));
-        const double b0 = -erf(er) / rm;
-        const double b1 = (b0 + a.eta * M_2_SQRTPI * e) / r2;
-        const double qj = a.q[j];
-        phi += qj * b0;
-        ex += qj * b1 * x;
-        ey += qj * b1 * y;
-        ez += qj * b1 * z;
-      }
-    }
-    if (a.do14) {
-      for (int n = a.p14_ptr[i]; n < a.p14_ptr[i + 1]; n++) {
-        const int j = a.p14_idx[n];
-        const int m = mi & a.mask[j];
-        double x = xi - a.r[3 * j], y = yi - a.r[3 * j + 1], z = zi - a.r[3 * j + 2];
-        min_image_ref(a.box, x, y, z);
-        const double r2 = x * x + y * y + z * z;
-        if (m & MMNB_SITE_HAS_Q) {
-          const double rs = a.rscreen[i] + a.rscreen[j];
-          double b0, b1;
-          if (r2 < rs * rs) {
-            b1 = 1.0 / (rs * rs * rs);
-            b0 = -0.5 * r2 * b1 + 1.5 / rs;
-          } else {
-            const double invr = 1.0 / sqrt(r2);
-            b0 = invr;
-            b1 = invr * invr * invr;
-          }
-          if (a.scale_e14) {
-            b0 *= a.e14;
-            b1 *= a.e14;
-          }
-          const double qj = a.q[j];
-          phi += qj * b0;
-          ex += qj * b1 * x;
-          ey += qj * b1 * y;
-          ez += qj * b1 * z;
-        }
-        if (m & MMNB_SITE_HAS_LJ) {
-          const double sg = a.geometric ? a.sig[i] * a.sig[j]
-                                        : (0.5 * (a.sig[i] + a.sig[j])) * (0.5 * (a.sig[i] + a.sig[j]));
-          const double s6 = sg * sg * sg;
-          const double b = 4 * sqrt(a.eps[i] * a.eps[j]) * s6;
-          const double aa = b * s6;
-          const double invr2 = 1.0 / r2;
-          const double invr6 = invr2 * invr2 * invr2;
-          double du = 12 * aa * invr6 * invr6 * invr2 - 6 * b * invr6 * invr2;
-          double u = aa * invr6 * invr6 - b * invr6;
-          if (a.scale_l14) {
-            u *= a.l14;
-            du *= a.l14;
-          }
-          elj += 0.5 * u;
-          vir += 0.5 * du * r2;
-          lx += du * x;
-          ly += du * y;
-          lz += du * z;
-        }
-      }
-    }
-    if (a.assign) {
-      // the same bits as adding to zeroed arrays (0 + x, which also turns -0 into +0)
-      a.phi[i] = 0.0 + phi;
-      a.evec[3 * i] = 0.0 + ex;
-      a.evec[3 * i + 1] = 0.0 + ey;
-      a.evec[3 * i + 2] = 0.0 + ez;
-      a.ljf[3 * i] = 0.0 + lx;
-      a.ljf[3 * i + 1] = 0.0 + ly;
-      a.ljf[3 * i + 2] = 0.0 + lz;
-    } else {
-      a.phi[i] += phi;
-      a.evec[3 * i] += ex;
-      a.evec[3 * i + 1] += ey;
-      a.evec[3 * i + 2] += ez;
-      if (a.do14) {
-        a.ljf[3 * i] += lx;
-        a.ljf[3 * i + 1] += ly;
-        a.ljf[3 * i + 2] += lz;
-      }
-    }
-  }
-  sl[threadIdx.x] = elj;
-  sv[threadIdx.x] = vir;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      sl[threadIdx.x] += sl[threadIdx.x + s];
-      sv[threadIdx.x] += sv[threadIdx.x + s];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    a.lj14_part[blockIdx.x] = sl[0];
-    if (a.vir14_part)
-      a.vir14_part[blockIdx.x] = sv[0];
-  }
+  sort_sites(r, q, sig, eps, rscreen, mask, sorted, group, ngroup, G, sr, sp, anchor, counter, flags);
+  build_rows(rows);
 }
 
 cudaError_t launch_sort_sites(mmnb_handle *h, const double *d_r)
 {
   const int n = h->ngroup * h->G;
-  k_sort_sites<<<div_up(n, 256), 256, 0, h->stream>>>(d_r, h->d_q, h->d_sig, h->d_eps, h->d_rscreen, h->d_mask,
+  k_sort_sites<<<sort_blocks(h, n), 32 * kRowWarps, 0, h->stream>>>(d_r, h->d_q, h->d_sig, h->d_eps, h->d_rscreen, h->d_mask,
                                                       h->d_sorted, h->d_group, h->ngroup, h->G, h->d_sr, h->d_sp,
-                                                      h->d_sanchor, h->d_wsum + 3, h->d_flags);
+                                                      h->d_sanchor, h->d_wsum + 3, h->d_flags, rebuild_args(h));
   h->launches += 1;
   return cudaGetLastError();
 }
-
-int pair_blocks(const mmnb_handle *h) { return div_up(h->ngroup, 4); }
-int excl_blocks(const mmnb_handle *h) { return div_up(h->nsite, kExclThreads); }
 
 template <bool SCREEN, bool GEXCL, bool VIR>
 static cudaError_t launch_pair64(mmnb_handle *h, PairArgs &a)
@@ -733,41 +607,6 @@ cudaError_t launch_rspace_fp64(mmnb_handle *h)
   if (h->has_rscreen)
     return h->any_gexcl ? launch_pair64<true, true, false>(h, a) : launch_pair64<true, false, false>(h, a);
   return h->any_gexcl ? launch_pair64<false, true, false>(h, a) : launch_pair64<false, false, false>(h, a);
-}
-
-cudaError_t launch_exclusions(mmnb_handle *h, const double *d_r)
-{
-  ExclArgs a;
-  a.nsite = h->nsite;
-  a.box = h->box;
-  a.eta = h->eta;
-  a.e14 = h->cfg.elec_1_4_scale_factor - 1;
-  a.l14 = h->cfg.lj_1_4_scale_factor - 1;
-  a.scale_e14 = fabs(h->cfg.elec_1_4_scale_factor - 1) > 1e-10;
-  a.scale_l14 = fabs(h->cfg.lj_1_4_scale_factor - 1) > 1e-10;
-  a.geometric = h->cfg.geometric_combining_for_sigma;
-  a.do14 = h->use_14 ? 1 : 0;
-  // the mixed form's pair kernels leave the FP64 site arrays alone: the
-  // exclusion corrections are their first write of an evaluation
-  a.assign = h->cfg.precision == MMNB_MIXED ? 1 : 0;
-  a.r = d_r;
-  a.q = h->d_q;
-  a.sig = h->d_sig;
-  a.eps = h->d_eps;
-  a.rscreen = h->d_rscreen;
-  a.mask = h->d_mask;
-  a.excl_ptr = h->d_excl_ptr;
-  a.excl_idx = h->d_excl_idx;
-  a.p14_ptr = h->d_p14_ptr;
-  a.p14_idx = h->d_p14_idx;
-  a.phi = h->d_phi;
-  a.evec = h->d_evec;
-  a.ljf = h->d_ljf;
-  a.lj14_part = h->d_lj_part + h->lj_pair_blocks;
-  a.vir14_part = h->want_virial ? h->d_vir_part + h->lj_pair_blocks : nullptr;
-  k_exclusions_fp64<<<excl_blocks(h), kExclThreads, 0, h->stream>>>(a);
-  h->launches += 1;
-  return cudaGetLastError();
 }
 
 }  // namespace mmnb

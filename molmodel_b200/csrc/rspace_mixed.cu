@@ -31,7 +31,7 @@
 // and an exclusion search per group pair: 494 us on 32^3 cells of solution (94,000
 // sites, groups of two to four); this layout 260 us (bound by issue, 63%; 290 us at 16 warps per SM, 260 at 24 with spills).
 
-#include "mmnb_internal.cuh"
+#include "nbrlist.cuh"
 
 namespace mmnb {
 
@@ -914,7 +914,7 @@ cudaError_t launch_rspace_water(mmnb_handle *h)
 // (sigma, sqrt(epsilon), rscreen, mask), padded with empty slots.  Rigid-water
 // layout (k_pair_water): per group three packed slots, (h1x, h2x, h1y, h2y),
 // (h1z, h2z, q1, q2), (qO, qO, sigma_O, sqrt(epsilon_O)).
-__global__ void k_prep_mixed(const double *__restrict__ r, const double *__restrict__ q,
+__device__ __forceinline__ void prep_mixed(const double *__restrict__ r, const double *__restrict__ q,
                              const double *__restrict__ sig, const double *__restrict__ eps,
                              const double *__restrict__ rscreen, const int *__restrict__ mask,
                              const int *__restrict__ sorted, const int *__restrict__ group, int ngroup, int G,
@@ -994,16 +994,29 @@ __global__ void k_prep_mixed(const double *__restrict__ r, const double *__restr
   }
 }
 
+__global__ void __launch_bounds__(32 * kRowWarps)
+k_prep_mixed(const double *__restrict__ r, const double *__restrict__ q, const double *__restrict__ sig,
+             const double *__restrict__ eps, const double *__restrict__ rscreen, const int *__restrict__ mask,
+             const int *__restrict__ sorted, const int *__restrict__ group, int ngroup, int G, int water,
+             float4 *__restrict__ site, float4 *__restrict__ par, double4 *__restrict__ anchor,
+             unsigned long long *__restrict__ wsum, int *__restrict__ flags, float4 *__restrict__ anc32, Box box,
+             int ncell, double3 edge, double3 inv_edge, RebuildArgs rows)
+{
+  prep_mixed(r, q, sig, eps, rscreen, mask, sorted, group, ngroup, G, water, site, par, anchor, wsum, flags, anc32,
+             box, ncell, edge, inv_edge);
+  build_rows(rows);
+}
+
 cudaError_t launch_prep_mixed(mmnb_handle *h, const double *d_r)
 {
   const int n = h->ngroup * h->G;
   const int water = h->water && !h->want_fields && h->cfg.include_rspace;
   const double3 edge = make_double3((float) h->cg.lc[0], (float) h->cg.lc[1], (float) h->cg.lc[2]);
   const double3 inv_edge = make_double3(1.0 / edge.x, 1.0 / edge.y, 1.0 / edge.z);
-  k_prep_mixed<<<div_up(n, 256), 256, 0, h->stream>>>(d_r, h->d_q, h->d_sig, h->d_eps, h->d_rscreen, h->d_mask,
+  k_prep_mixed<<<sort_blocks(h, n), 32 * kRowWarps, 0, h->stream>>>(d_r, h->d_q, h->d_sig, h->d_eps, h->d_rscreen, h->d_mask,
                                                       h->d_sorted, h->d_group, h->ngroup, h->G, water, h->mx.site,
                                                       h->mx.par, h->mx.anchor, h->d_wsum, h->d_flags, h->mx.anc32,
-                                                      h->box, h->cg.n, edge, inv_edge);
+                                                      h->box, h->cg.n, edge, inv_edge, rebuild_args(h));
   h->launches += 1;
   return cudaGetLastError();
 }

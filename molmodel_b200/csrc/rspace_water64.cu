@@ -42,7 +42,7 @@
 // four copies.  On one row per warp the table's copy-in shows: asynchronous, 21 -> 17
 // us on 216 waters.
 
-#include "mmnb_internal.cuh"
+#include "nbrlist.cuh"
 
 #include <algorithm>
 
@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(kW64Warps * 32, 1) k_pair_water64(Water64Args 
 // (h1x, h1y, h1z, h2x), (h2y, h2z, qO, qH1), (qH2, sigma_O, sqrt(eps_O), 0) with
 // the H positions taken from the anchor O; the row counter is cleared and a
 // non-finite coordinate is flagged.
-__global__ void k_sort_water64(const double *__restrict__ r, const double *__restrict__ q,
+__device__ __forceinline__ void sort_water64(const double *__restrict__ r, const double *__restrict__ q,
                                const double *__restrict__ sig, const double *__restrict__ eps,
                                const int *__restrict__ sorted, const int *__restrict__ group, int ngroup,
                                double4 *__restrict__ anchor, double2 *__restrict__ rec,
@@ -380,11 +380,21 @@ __global__ void k_sort_water64(const double *__restrict__ r, const double *__res
   o[5] = make_double2(sqrt(eps[a0]), 0.0);
 }
 
+__global__ void __launch_bounds__(32 * kRowWarps)
+k_sort_water64(const double *__restrict__ r, const double *__restrict__ q, const double *__restrict__ sig,
+               const double *__restrict__ eps, const int *__restrict__ sorted, const int *__restrict__ group,
+               int ngroup, double4 *__restrict__ anchor, double2 *__restrict__ rec,
+               unsigned long long *__restrict__ counter, int *__restrict__ flags, RebuildArgs rows)
+{
+  sort_water64(r, q, sig, eps, sorted, group, ngroup, anchor, rec, counter, flags);
+  build_rows(rows);
+}
+
 cudaError_t launch_sort_water64(mmnb_handle *h, const double *d_r)
 {
-  k_sort_water64<<<div_up(h->ngroup, 256), 256, 0, h->stream>>>(
+  k_sort_water64<<<sort_blocks(h, h->ngroup), 32 * kRowWarps, 0, h->stream>>>(
       d_r, h->d_q, h->d_sig, h->d_eps, h->d_sorted, h->d_group, h->ngroup, h->d_sp, reinterpret_cast<double2 *>(h->d_sr), h->d_wsum + 3,
-      h->d_flags);
+      h->d_flags, rebuild_args(h));
   h->launches += 1;
   return cudaGetLastError();
 }

@@ -166,22 +166,11 @@ extern "C" int mmnb_virial(mmnb_handle *h, const double *r, int nmol, const int 
     return s;
   if (e)
     *e = en;
-  // X's partial sums: per row (FP64 water kernel), per block (other kernels,
-  // then the exclusion kernel's 1-4 LJ blocks), or one fixed-point word
-  // (mixed water kernel)
-  const double *part = h->d_vir_part;
-  int npart = 0;
-  const unsigned long long *fixed = nullptr;
-  if (h->cfg.include_rspace) {
-    if (h->used_rows64) {
-      part = h->d_vir_row;
-      npart = h->ngroup;
-    } else if (h->used_fx) {
-      fixed = h->d_wsum + 4;
-    } else {
-      npart = h->lj_pair_blocks;
-    }
-  }
+  // X's sums: per row (FP64 pair kernels) or one fixed-point word (mixed pair
+  // kernels), and the 1-4 LJ pairs' sum (intramolecular: they add to X)
+  const double *part = h->d_vir_row;
+  const int npart = h->cfg.include_rspace && h->used_rows64 ? h->ngroup : 0;
+  const unsigned long long *fixed = h->cfg.include_rspace && h->used_fx ? h->d_wsum + 4 : nullptr;
   double *res = h->d_vir_molw + nmol;
   k_virial_mol<<<div_up(nmol, kVirThreads), kVirThreads, 0, h->stream>>>(nmol, h->d_vir_mol, h->d_vir_mass,
                                                                          h->d_r, h->d_f, h->d_vir_molw);
@@ -191,17 +180,10 @@ extern "C" int mmnb_virial(mmnb_handle *h, const double *r, int nmol, const int 
   if ((ce = cudaGetLastError()) != cudaSuccess ||
       (ce = cudaMemcpyAsync(out, res, sizeof(double) * 2, cudaMemcpyDeviceToHost, h->stream)) != cudaSuccess)
     return vir_fail(h, MMNB_ERR_CUDA, cudaGetErrorString(ce));
-  if (h->cfg.include_rspace && h->use_14) {
-    // the 1-4 LJ terms of the exclusion kernel (intramolecular: they add to X)
-    std::vector<double> p14(h->lj_excl_blocks);
-    if ((ce = cudaMemcpyAsync(p14.data(), h->d_vir_part + h->lj_pair_blocks, sizeof(double) * p14.size(),
-                              cudaMemcpyDeviceToHost, h->stream)) != cudaSuccess)
-      return vir_fail(h, MMNB_ERR_CUDA, cudaGetErrorString(ce));
-    if ((ce = cudaStreamSynchronize(h->stream)) != cudaSuccess)
-      return vir_fail(h, MMNB_ERR_CUDA, cudaGetErrorString(ce));
-    for (double v : p14)
-      out[2] += v;
-  }
+  if (h->cfg.include_rspace && h->use_14 &&
+      (ce = cudaMemcpyAsync(out + 2, h->d_energy + 8, sizeof(double), cudaMemcpyDeviceToHost, h->stream)) !=
+          cudaSuccess)
+    return vir_fail(h, MMNB_ERR_CUDA, cudaGetErrorString(ce));
   if ((ce = cudaStreamSynchronize(h->stream)) != cudaSuccess)
     return vir_fail(h, MMNB_ERR_CUDA, cudaGetErrorString(ce));
   *w = out[0] - en.elec - (out[1] + out[2]) - 3 * en.lj_correction;
