@@ -413,7 +413,7 @@ static int grad_p3m_scratch(mmnb_handle *h, P3mScratch &s)
 {
   const size_t nr = (size_t) h->mesh[0] * h->mesh[1] * h->mesh[2];
   const size_t nk = (size_t) h->mesh[0] * h->mesh[1] * (h->mesh[2] / 2 + 1);
-  if (h->plan_r2c) {
+  if (h->cfg.precision != MMNB_MIXED) {
     s.r2c = h->plan_r2c;
     s.c2r = h->plan_c2r;
     if (h->cfg.p3m_ik_differentiate) {
@@ -429,7 +429,7 @@ static int grad_p3m_scratch(mmnb_handle *h, P3mScratch &s)
   }
   // ik: three spread meshes and the summed spectrum's mesh
   const int nm = h->cfg.p3m_ik_differentiate ? 4 : 1;
-  if (!h->gplan_r2c) {
+  if (!h->d_gmesh) {
     cudaError_t e = cudaMalloc(&h->d_gmesh, sizeof(double) * nr * nm);
     if (e == cudaSuccess)
       e = cudaMalloc(&h->d_gmeshk, sizeof(cufftDoubleComplex) * nk * nm);
@@ -437,8 +437,9 @@ static int grad_p3m_scratch(mmnb_handle *h, P3mScratch &s)
       h->err = std::string("gradient mesh: ") + cudaGetErrorString(e);
       return MMNB_ERR_CUDA;
     }
-    if (cufftPlan3d(&h->gplan_r2c, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_D2Z) != CUFFT_SUCCESS ||
-        cufftPlan3d(&h->gplan_c2r, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_Z2D) != CUFFT_SUCCESS) {
+    const bool own = h->d_fft64 && nm == 1;
+    if (!own && (cufftPlan3d(&h->gplan_r2c, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_D2Z) != CUFFT_SUCCESS ||
+        cufftPlan3d(&h->gplan_c2r, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_Z2D) != CUFFT_SUCCESS)) {
       h->err = "gradient mesh: cuFFT plan";
       return MMNB_ERR_CUDA;
     }

@@ -4,6 +4,7 @@
 
 #include <atomic>
 
+#include "meshfft.cuh"
 #include "mmnb_internal.cuh"
 
 #include <algorithm>
@@ -428,6 +429,17 @@ int setup_p3m(mmnb_handle *h)
   const size_t nr = (size_t) h->mesh[0] * h->mesh[1] * h->mesh[2];
   const size_t nk = (size_t) h->mesh[0] * h->mesh[1] * (h->mesh[2] / 2 + 1);
   int s;
+  // ik on a mesh of odd point count stays with the plans, which refuse it (the field
+  // meshes follow one another unaligned)
+  if (!(c.p3m_ik_differentiate && nr % 2))
+    for (int bytes : {4, 8})
+      if (mesh_fft_fits(h->mesh, bytes)) {
+        void *&table = bytes == 4 ? h->d_fft32 : h->d_fft64;
+        std::vector<double> w(2 * mesh_fft_table_size(h->mesh));
+        mesh_fft_table(h->mesh, bytes, w.data());
+        CK(cudaMalloc(&table, 16 * mesh_fft_table_size(h->mesh)));
+        CK(cudaMemcpy(table, w.data(), 2 * bytes * mesh_fft_table_size(h->mesh), cudaMemcpyHostToDevice));
+      }
   if ((s = dalloc(h, &h->d_green, nk)) || (s = dalloc(h, &h->d_kvec, 3 * nk)) ||
       (s = dalloc(h, &h->d_chi_part, (nk + 127) / 128)))
     return s;
@@ -439,17 +451,22 @@ int setup_p3m(mmnb_handle *h)
     if (c.p3m_ik_differentiate)
       if ((s = dalloc(h, &h->d_egrid32, 3 * nr)) || (s = dalloc(h, &h->d_egridk32, 3 * nk)))
         return s;
-    CKFFT(cufftPlan3d(&h->plan_r2c32, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_R2C));
-    CKFFT(cufftPlan3d(&h->plan_c2r32, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_C2R));
-    CKFFT(cufftSetStream(h->plan_r2c32, h->stream));
-    CKFFT(cufftSetStream(h->plan_c2r32, h->stream));
+    if (!h->d_fft32) {
+      CKFFT(cufftPlan3d(&h->plan_r2c32, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_R2C));
+      CKFFT(cufftPlan3d(&h->plan_c2r32, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_C2R));
+      CKFFT(cufftSetStream(h->plan_r2c32, h->stream));
+      CKFFT(cufftSetStream(h->plan_c2r32, h->stream));
+    }
   } else {
     if ((s = dalloc(h, &h->d_mesh, nr * (c.p3m_ik_differentiate ? 1 : 1))) || (s = dalloc(h, &h->d_meshk, nk)))
       return s;
-    CKFFT(cufftPlan3d(&h->plan_r2c, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_D2Z));
-    CKFFT(cufftPlan3d(&h->plan_c2r, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_Z2D));
-    CKFFT(cufftSetStream(h->plan_r2c, h->stream));
-    CKFFT(cufftSetStream(h->plan_c2r, h->stream));
+    // (the charge gradients' dipole solve with ik transforms three meshes: plans)
+    if (!h->d_fft64 || c.p3m_ik_differentiate) {
+      CKFFT(cufftPlan3d(&h->plan_r2c, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_D2Z));
+      CKFFT(cufftPlan3d(&h->plan_c2r, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_Z2D));
+      CKFFT(cufftSetStream(h->plan_r2c, h->stream));
+      CKFFT(cufftSetStream(h->plan_c2r, h->stream));
+    }
     if (c.p3m_ik_differentiate)
       if ((s = dalloc(h, &h->d_egrid, 3 * nr)) || (s = dalloc(h, &h->d_egridk, 3 * nk)))
         return s;
@@ -498,7 +515,8 @@ void free_all(mmnb_handle *h)
                   h->d_top2, h->d_nbr, h->d_nbr_count, h->d_pnbr, h->d_pcount, h->d_plast, h->d_flags, h->d_sr,
                   h->d_sp, h->d_sanchor, h->d_site_of_slot,
                   h->d_phi, h->d_evec, h->d_ljf, h->d_site_part, h->d_energy, h->d_r, h->d_f,
-                  h->d_mesh, h->d_meshk, h->d_green, h->d_kvec, h->d_egrid, h->d_egridk, h->d_mesh32,
+                  h->d_fft32, h->d_fft64, h->d_mesh, h->d_meshk, h->d_green, h->d_kvec, h->d_egrid,
+                  h->d_egridk, h->d_mesh32,
                   h->d_meshk32, h->d_green32, h->d_egrid32, h->d_egridk32, h->d_mesh_fx,
                   h->mx.site, h->mx.par, h->mx.anchor, h->mx.anc32, h->mx.acc, h->d_wsum,
                   h->d_bwd, h->d_esp, h->d_gmesh, h->d_gmeshk, h->d_chi_part};

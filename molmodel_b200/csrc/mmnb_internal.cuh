@@ -236,6 +236,9 @@ struct mmnb_handle {
   // P3M
   bool p3m = false;
   int mesh[3] = {0, 0, 0};
+  // the mesh solve's own transforms (meshfft.cu) where they take the mesh: twiddle
+  // factors of the FP32 and FP64 forms (null: the plans below)
+  void *d_fft32 = nullptr, *d_fft64 = nullptr;
   cufftHandle plan_r2c = 0, plan_c2r = 0;
   double *d_mesh = nullptr;
   cufftDoubleComplex *d_meshk = nullptr;
@@ -327,7 +330,7 @@ cudaError_t launch_p3m_fp64(mmnb_handle *h, const double *d_r);
 struct P3mScratch {
   double *spread = nullptr, *solve = nullptr;
   cufftDoubleComplex *spreadk = nullptr, *solvek = nullptr;
-  cufftHandle r2c = 0, c2r = 0;
+  cufftHandle r2c = 0, c2r = 0;  // or none: own transforms
 };
 // d_psi += mesh potential of the dipoles q_j g_j (g: 3 per site), FP64
 cudaError_t launch_p3m_dipole_fp64(mmnb_handle *h, const double *d_r, const double *d_g, const P3mScratch &s,

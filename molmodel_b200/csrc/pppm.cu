@@ -15,6 +15,7 @@
 // once per box on the GPU in FP64.
 
 #include "mesh.cuh"
+#include "meshfft.cuh"
 
 namespace mmnb {
 
@@ -223,6 +224,15 @@ static int lane_blocks(int nsite)
   return div_up((long) div_up(nsite, 32 / P) * 32, 128);
 }
 
+static cudaError_t mesh_solve64(mmnb_handle *h, double *in, cufftDoubleComplex *spec, cufftDoubleComplex *fspec,
+                                double *out, double *fout)
+{
+  MeshSolve<double> m = {{h->mesh[0], h->mesh[1], h->mesh[2]}, h->d_fft64, h->d_green, h->d_kvec, spec, fspec,
+                         out, fout};
+  h->launches += 3;
+  return mesh_solve(m, in, h->stream);
+}
+
 // charge assignment and the FFT round trip
 template <int P>
 static cudaError_t p3m_fp64_p(mmnb_handle *h, const double *d_r)
@@ -236,6 +246,12 @@ static cudaError_t p3m_fp64_p(mmnb_handle *h, const double *d_r)
     return e;
   k_spread_fp64<P><<<lane_blocks<P>(h->nsite), 128, 0, h->stream>>>(m, d_r, h->d_q, h->d_mask, h->d_mesh);
   timing_mark(h, "p3m_spread");
+  h->launches += 1;
+  if (h->d_fft64) {
+    e = mesh_solve64(h, h->d_mesh, h->d_meshk, h->d_egridk, h->d_mesh, h->d_egrid);
+    timing_mark(h, "p3m_fft");
+    return e;
+  }
   if (cufftSetStream(h->plan_r2c, h->stream) != CUFFT_SUCCESS ||
       cufftSetStream(h->plan_c2r, h->stream) != CUFFT_SUCCESS ||
       cufftExecD2Z(h->plan_r2c, h->d_mesh, h->d_meshk) != CUFFT_SUCCESS)
@@ -249,7 +265,7 @@ static cudaError_t p3m_fp64_p(mmnb_handle *h, const double *d_r)
   if (cufftExecZ2D(h->plan_c2r, h->d_meshk, h->d_mesh) != CUFFT_SUCCESS)
     return cudaErrorUnknown;
   timing_mark(h, "p3m_fft");
-  h->launches += 2;
+  h->launches += 1;
   return cudaGetLastError();
 }
 
@@ -380,6 +396,14 @@ static cudaError_t p3m_dipole_p(mmnb_handle *h, const double *d_r, const double 
     return e;
   k_spread_dipole_fp64<P><<<lane_blocks<P>(h->nsite), 128, 0, h->stream>>>(m, d_r, h->d_q, h->d_mask, d_g, ik, nr,
                                                                          s.spread);
+  if (!s.r2c) {
+    e = mesh_solve64(h, s.spread, s.spreadk, nullptr, s.solve, nullptr);
+    if (e != cudaSuccess)
+      return e;
+    k_gather_potential_fp64<P><<<lane_blocks<P>(h->nsite), 128, 0, h->stream>>>(m, d_r, s.solve, d_psi);
+    h->launches += 2;
+    return cudaGetLastError();
+  }
   if (cufftSetStream(s.r2c, h->stream) != CUFFT_SUCCESS || cufftSetStream(s.c2r, h->stream) != CUFFT_SUCCESS)
     return cudaErrorUnknown;
   for (int d = 0; d < nmesh; d++)
@@ -627,6 +651,15 @@ static cudaError_t p3m_mixed_p(mmnb_handle *h, const double *d_r, bool assigned)
   const long nk = (long) h->mesh[0] * h->mesh[1] * (h->mesh[2] / 2 + 1);
   if (!assigned)
     spread_mixed_p<P>(h, m, d_r, 0, h->nsite);
+  if (h->d_fft32) {
+    timing_mark(h, "p3m_spread");
+    MeshSolve<float> ms = {{h->mesh[0], h->mesh[1], h->mesh[2]}, h->d_fft32, h->d_green32, h->d_kvec, h->d_meshk32,
+                           h->d_egridk32, h->d_mesh32, h->d_egrid32};
+    const cudaError_t e = mesh_solve(ms, h->d_mesh_fx, h->stream);
+    timing_mark(h, "p3m_fft");
+    h->launches += 3;
+    return e;
+  }
   k_mesh_fx_to_f32<<<div_up((long) nr, 256), 256, 0, h->stream>>>(nr, h->d_mesh_fx, h->d_mesh32);
   timing_mark(h, "p3m_spread");
   if (cufftSetStream(h->plan_r2c32, h->stream) != CUFFT_SUCCESS ||
