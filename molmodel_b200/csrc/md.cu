@@ -13,9 +13,10 @@
 // Their results are the constraint solutions the reference's iterations
 // converge to.
 //
-// The step (force zeroing, the two half kicks with their constraints, the
-// evaluation and the energy record) is captured once into a CUDA graph and
-// replayed; kinetic energy is reduced per block and summed in index order by
+// A run drifts once, then replays one CUDA graph per step: the evaluation, and a kernel
+// with the second half kick, its constraint, the energy record and, but for the run's
+// last step, the next step's first half kick, drift and constraint (a kernel less per
+// step, and the forces read once); kinetic energy is reduced per block and summed in index order by
 // the last block, and each step's (kinetic, potential, conserved) energies are
 // appended to a device log that is read back once per run.
 
@@ -45,7 +46,7 @@ struct mmnb_md {
   double *d_energy = nullptr;   // the evaluation's energies (elec, lj, tail, total)
   double *d_ke_part = nullptr;  // per block
   double *d_log = nullptr;      // 3 per step
-  unsigned long long *d_ctl = nullptr;  // [0] finished-block counter, [1] log position
+  unsigned long long *d_ctl = nullptr;  // [0] finished-block counter, [1] log position, [2] steps of the run
   int log_cap = 0;
   int ke_blocks = 0;
   cudaGraph_t graph = nullptr;
@@ -70,7 +71,7 @@ struct mmnb_md_batch {
 
 namespace mmnb {
 
-constexpr int kMdThreads = 256;
+constexpr int kMdThreads = 64;  // FP64 chains: few warps an SM
 
 __global__ void k_md_scale(double *__restrict__ v, int n, double s)
 {
@@ -182,27 +183,19 @@ __device__ void settle_velocities(const MdArgs &a, V3 ra_, V3 rb_, V3 rc_, V3 &v
   vc = vc + ih * (-1.0 * m2 * uac - m3 * ubc);
 }
 
-// first half kick, drift, position constraint (one thread per molecule, or
-// per site without constraints)
-__global__ void k_md_drift(MdArgs a)
+// first half kick, drift, position constraint of site t (no constraints) or molecule t
+__device__ __forceinline__ void drift_site(const MdArgs &a, int t, V3 v, V3 f)
 {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const double hdt = 0.5 * a.dt;
-  if (!a.rigid) {
-    if (t >= a.nsite)
-      return;
-    V3 v = ld3(a.v + 3 * t) + (hdt * a.minv[t]) * ld3(a.f + 3 * t);
-    st3(a.v + 3 * t, v);
-    st3(a.r + 3 * t, ld3(a.r + 3 * t) + a.dt * v);
-    return;
-  }
-  if (t >= a.nmol)
-    return;
+  v = v + (0.5 * a.dt * a.minv[t]) * f;
+  st3(a.v + 3 * t, v);
+  st3(a.r + 3 * t, ld3(a.r + 3 * t) + a.dt * v);
+}
+__device__ __forceinline__ void drift_water(const MdArgs &a, int t, const V3 (&x0)[3], V3 (&v)[3], const V3 (&f)[3])
+{
   const int s = 3 * t;
-  V3 x0[3], x1[3], v[3];
+  V3 x1[3];
   for (int k = 0; k < 3; k++) {
-    x0[k] = ld3(a.r + 3 * (s + k));
-    v[k] = ld3(a.v + 3 * (s + k)) + (hdt * a.minv[s + k]) * ld3(a.f + 3 * (s + k));
+    v[k] = v[k] + (0.5 * a.dt * a.minv[s + k]) * f[k];
     x1[k] = x0[k] + a.dt * v[k];
   }
   V3 y[3] = {x1[0], x1[1], x1[2]};
@@ -212,6 +205,31 @@ __global__ void k_md_drift(MdArgs a)
     st3(a.r + 3 * (s + k), y[k]);
     st3(a.v + 3 * (s + k), v[k] + idt * (y[k] - x1[k]));
   }
+}
+
+// a run's first drift, of up to kMdListMax integrators (blockIdx.y)
+constexpr int kMdListMax = 16;
+struct MdList {
+  MdArgs a[kMdListMax];
+};
+__global__ void __launch_bounds__(kMdThreads) k_md_drift(MdList list)
+{
+  const MdArgs &a = list.a[blockIdx.y];
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (a.rigid ? a.nmol : a.nsite))
+    return;
+  if (!a.rigid) {
+    drift_site(a, t, ld3(a.v + 3 * t), ld3(a.f + 3 * t));
+    return;
+  }
+  V3 x[3], v[3], f[3];
+  for (int k = 0; k < 3; k++) {
+    const int i = 3 * (3 * t + k);
+    x[k] = ld3(a.r + i);
+    v[k] = ld3(a.v + i);
+    f[k] = ld3(a.f + i);
+  }
+  drift_water(a, t, x, v, f);
 }
 
 __device__ __forceinline__ double md_block_sum(double x, double *sh)
@@ -226,32 +244,44 @@ __device__ __forceinline__ double md_block_sum(double x, double *sh)
   return sh[0];
 }
 
-// second half kick, velocity constraint, kinetic energy and the step's record
+// Second half kick, velocity constraint, kinetic energy and the step's record; then the
+// next step's drift unless the run ends with this step.  (kick = 0: the velocity
+// constraint alone, of a new state.)  The log position says which step this is: the
+// last block advances it, after every block has read it.
 __global__ void __launch_bounds__(kMdThreads) k_md_kick(MdArgs a, int kick)
 {
   __shared__ double sh[kMdThreads];
   __shared__ bool last;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool drift = kick && a.ctl[1] + 1 < a.ctl[2];
   const double hdt = kick ? 0.5 * a.dt : 0.0;
   double ke = 0;
   if (!a.rigid) {
     if (t < a.nsite) {
-      V3 v = ld3(a.v + 3 * t) + (hdt * a.minv[t]) * ld3(a.f + 3 * t);
-      st3(a.v + 3 * t, v);
+      const V3 f = ld3(a.f + 3 * t);
+      V3 v = ld3(a.v + 3 * t) + (hdt * a.minv[t]) * f;
       ke = 0.5 * a.m[t] * dot(v, v);
+      if (drift)
+        drift_site(a, t, v, f);
+      else
+        st3(a.v + 3 * t, v);
     }
   } else if (t < a.nmol) {
     const int s = 3 * t;
-    V3 x[3], v[3];
+    V3 x[3], v[3], f[3];
     for (int k = 0; k < 3; k++) {
       x[k] = ld3(a.r + 3 * (s + k));
-      v[k] = ld3(a.v + 3 * (s + k)) + (hdt * a.minv[s + k]) * ld3(a.f + 3 * (s + k));
+      f[k] = ld3(a.f + 3 * (s + k));
+      v[k] = ld3(a.v + 3 * (s + k)) + (hdt * a.minv[s + k]) * f[k];
     }
     settle_velocities(a, x[0], x[1], x[2], v[0], v[1], v[2]);
-    for (int k = 0; k < 3; k++) {
-      st3(a.v + 3 * (s + k), v[k]);
+    for (int k = 0; k < 3; k++)
       ke += 0.5 * a.m[s + k] * dot(v[k], v[k]);
-    }
+    if (drift)
+      drift_water(a, t, x, v, f);
+    else
+      for (int k = 0; k < 3; k++)
+        st3(a.v + 3 * (s + k), v[k]);
   }
   const double bs = md_block_sum(ke, sh);
   if (threadIdx.x == 0) {
@@ -295,11 +325,12 @@ struct MdIo {
   const double *log[kMdIoMax];
 };
 
-__global__ void k_md_begin(MdIo io)
+__global__ void k_md_begin(MdIo io, int nsteps)
 {
   const int t = threadIdx.x;
   if (t < io.n) {
     io.ctl[t][1] = 0ull;
+    io.ctl[t][2] = nsteps;
     io.flags[t][kFlagOverflow] = 0;
   }
 }
@@ -319,6 +350,31 @@ __global__ void k_md_report(MdIo io, int nlog, double *__restrict__ out)
 
 using namespace mmnb;
 
+static MdArgs md_args(mmnb_md *md, double *log)
+{
+  MdArgs a;
+  a.nsite = md->nsite;
+  a.nmol = md->nmol;
+  a.rigid = md->rigid;
+  a.dt = md->dt;
+  a.m_o = md->m_o;
+  a.m_h = md->m_h;
+  a.ra = md->ra;
+  a.rb = md->rb;
+  a.rc = md->rc;
+  a.r = md->d_r;
+  a.v = md->d_v;
+  a.f = md->d_f;
+  a.minv = md->d_minv;
+  a.m = md->d_m;
+  a.energy = md->d_energy;
+  a.ke_part = md->d_ke_part;
+  a.log = log;
+  a.ctl = md->d_ctl;
+  a.log_cap = md->log_cap;
+  return a;
+}
+
 // integrators [lo, ...) of a run, as many as one launch takes
 static MdIo md_io(mmnb_md *const *md, size_t n, size_t lo)
 {
@@ -332,10 +388,21 @@ static MdIo md_io(mmnb_md *const *md, size_t n, size_t lo)
   return io;
 }
 
-static cudaError_t md_begin(mmnb_md *const *md, size_t n, cudaStream_t s)
+// clears and the first drift
+static cudaError_t md_begin(mmnb_md *const *md, size_t n, int nsteps, cudaStream_t s)
 {
   for (size_t lo = 0; lo < n; lo += kMdIoMax)
-    k_md_begin<<<1, kMdIoMax, 0, s>>>(md_io(md, n, lo));
+    k_md_begin<<<1, kMdIoMax, 0, s>>>(md_io(md, n, lo), nsteps);
+  for (size_t lo = 0; lo < n; lo += kMdListMax) {
+    MdList list;
+    int blocks = 0;
+    const int m = (int) std::min<size_t>(kMdListMax, n - lo);
+    for (int i = 0; i < m; i++) {
+      list.a[i] = md_args(md[lo + i], nullptr);
+      blocks = std::max(blocks, md[lo + i]->ke_blocks);
+    }
+    k_md_drift<<<dim3(blocks, m), kMdThreads, 0, s>>>(list);
+  }
   return cudaGetLastError();
 }
 
@@ -400,31 +467,6 @@ static int md_fail(mmnb_md *md, int code, const std::string &msg)
       return md_fail(md, MMNB_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
-static MdArgs md_args(mmnb_md *md, double *log)
-{
-  MdArgs a;
-  a.nsite = md->nsite;
-  a.nmol = md->nmol;
-  a.rigid = md->rigid;
-  a.dt = md->dt;
-  a.m_o = md->m_o;
-  a.m_h = md->m_h;
-  a.ra = md->ra;
-  a.rb = md->rb;
-  a.rc = md->rc;
-  a.r = md->d_r;
-  a.v = md->d_v;
-  a.f = md->d_f;
-  a.minv = md->d_minv;
-  a.m = md->d_m;
-  a.energy = md->d_energy;
-  a.ke_part = md->d_ke_part;
-  a.log = log;
-  a.ctl = md->d_ctl;
-  a.log_cap = md->log_cap;
-  return a;
-}
-
 extern "C" {
 
 int mmnb_md_create(mmnb_handle *h, const double *site_mass, double dt, int rigid_water, double r_oh,
@@ -478,10 +520,10 @@ int mmnb_md_create(mmnb_handle *h, const double *site_mass, double dt, int rigid
       cudaMalloc(&md->d_minv, h->nsite * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&md->d_energy, 8 * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&md->d_ke_part, md->ke_blocks * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&md->d_ctl, 2 * sizeof(unsigned long long)) != cudaSuccess ||
+      cudaMalloc(&md->d_ctl, 3 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMemcpy(md->d_m, m.data(), h->nsite * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(md->d_minv, minv.data(), h->nsite * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemset(md->d_ctl, 0, 2 * sizeof(unsigned long long)) != cudaSuccess ||
+      cudaMemset(md->d_ctl, 0, 3 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMemset(md->d_v, 0, n3 * sizeof(double)) != cudaSuccess) {
     mmnb_md_destroy(md);
     return MMNB_ERR_CUDA;
@@ -503,7 +545,7 @@ int mmnb_md_set_state(mmnb_md *md, const double *r, const double *v)
     MDCK(cudaMemsetAsync(md->d_v, 0, n3 * sizeof(double), h->stream));
   // velocities obey the constraints before the first step (the positions
   // are taken as given: a rigid triangle)
-  MDCK(cudaMemsetAsync(md->d_ctl, 0, 2 * sizeof(unsigned long long), h->stream));
+  MDCK(cudaMemsetAsync(md->d_ctl, 0, 3 * sizeof(unsigned long long), h->stream));
   const MdArgs a = md_args(md, nullptr);
   k_md_kick<<<md->ke_blocks, kMdThreads, 0, h->stream>>>(a, 0);
   MDCK(cudaGetLastError());
@@ -515,7 +557,7 @@ int mmnb_md_set_state(mmnb_md *md, const double *r, const double *v)
   if (s)
     return md_fail(md, s, mmnb_last_error(h));
   MDCK(cudaMemcpyAsync(md->d_f, f.data(), n3 * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  MDCK(cudaMemsetAsync(md->d_ctl, 0, 2 * sizeof(unsigned long long), h->stream));
+  MDCK(cudaMemsetAsync(md->d_ctl, 0, 3 * sizeof(unsigned long long), h->stream));
   MDCK(cudaStreamSynchronize(h->stream));
   return MMNB_OK;
 }
@@ -525,8 +567,6 @@ static int md_record(mmnb_md *md, double *log)
 {
   mmnb_handle *h = md->h;
   const MdArgs a = md_args(md, log);
-  const int n = md->rigid ? md->nmol : md->nsite;
-  k_md_drift<<<div_up(n, 128), 128, 0, h->stream>>>(a);
   h->assign_forces = true;
   const int s = mmnb_compute_device(h, md->d_r, md->d_f, md->d_energy);
   h->assign_forces = false;
@@ -604,7 +644,7 @@ int mmnb_md_run(mmnb_md *md, int nsteps, double *energies)
     if (s)
       return s;
   }
-  MDCK(md_begin(&md, 1, h->stream));
+  MDCK(md_begin(&md, 1, nsteps, h->stream));
   for (int i = 0; i < nsteps; i++)
     MDCK(cudaGraphLaunch(md->exec, h->stream));
   MDCK(md_end(md->report, &md, 1, nsteps, energies ? &energies : nullptr, h->stream));
@@ -790,7 +830,7 @@ int mmnb_md_batch_run(mmnb_md_batch *b, int nsteps, double *const *energies)
   }
   const size_t n = b->md.size();
   if (e == cudaSuccess)
-    e = md_begin(b->md.data(), n, b->master);
+    e = md_begin(b->md.data(), n, nsteps, b->master);
   for (int i = 0; i < nsteps && e == cudaSuccess; i++)
     e = cudaGraphLaunch(b->exec, b->master);
   if (e == cudaSuccess)
