@@ -252,6 +252,7 @@ __global__ void __launch_bounds__(kMdThreads) k_md_kick(MdArgs a, int kick)
 {
   __shared__ double sh[kMdThreads];
   __shared__ bool last;
+  after_previous();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const bool drift = kick && a.ctl[1] + 1 < a.ctl[2];
   const double hdt = kick ? 0.5 * a.dt : 0.0;
@@ -572,8 +573,7 @@ static int md_record(mmnb_md *md, double *log)
   h->assign_forces = false;
   if (s)
     return md_fail(md, s, mmnb_last_error(h));
-  k_md_kick<<<md->ke_blocks, kMdThreads, 0, h->stream>>>(a, 1);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_after(h, k_md_kick, md->ke_blocks, kMdThreads, 0, a, 1);
   if (e != cudaSuccess)
     return md_fail(md, MMNB_ERR_CUDA, cudaGetErrorString(e));
   return MMNB_OK;

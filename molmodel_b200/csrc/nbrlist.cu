@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(kCheckThreads) k_list_check(const double *__re
   __shared__ double sa[kCheckThreads], sb[kCheckThreads];
   __shared__ bool last_block;
   double a = 0, b = 0, pa = 0, pb = 0;
+  cudaTriggerProgrammaticLaunchCompletion();
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ngroup; g += gridDim.x * blockDim.x) {
     const int s0 = group[2 * g];
     const double x = r[3 * s0], y = r[3 * s0 + 1], z = r[3 * s0 + 2];
@@ -311,6 +312,7 @@ __device__ int sort_cells(const RebuildArgs &a, int c0, int base, int *warp_tot)
 // steps, 98,304 sites mixed 186 -> 178 us.
 __global__ void __launch_bounds__(kCellThreads) k_list_assign(RebuildArgs a)
 {
+  after_previous();
   if (!a.flags[kFlagRebuild])
     return;
   const int g = blockIdx.x * kCellThreads + threadIdx.x;
@@ -320,6 +322,7 @@ __global__ void __launch_bounds__(kCellThreads) k_list_assign(RebuildArgs a)
 
 __global__ void __launch_bounds__(kCellThreads) k_list_sort(RebuildArgs a)
 {
+  after_previous();
   if (!a.flags[kFlagRebuild])
     return;
   __shared__ int warp_tot[kCellThreads / 32];
@@ -336,6 +339,7 @@ __global__ void __launch_bounds__(kCellThreads) k_list_sort(RebuildArgs a)
 // both steps by one block, for boxes it handles as fast as two launches would
 __global__ void __launch_bounds__(kOneBlockThreads) k_list_cells(RebuildArgs a)
 {
+  after_previous();
   if (!a.flags[kFlagRebuild])
     return;
   __shared__ int warp_tot[kOneBlockThreads / 32];
@@ -420,11 +424,11 @@ cudaError_t launch_list_cells(mmnb_handle *h)
 {
   const RebuildArgs a = rebuild_args(h);
   if (h->ngroup <= kOneBlockGroups) {
-    k_list_cells<<<1, kOneBlockThreads, 0, h->stream>>>(a);
+    launch_after(h, k_list_cells, 1, kOneBlockThreads, 0, a);
     h->launches += 1;
   } else {
-    k_list_assign<<<div_up(h->ngroup, kCellThreads), kCellThreads, 0, h->stream>>>(a);
-    k_list_sort<<<div_up(h->ncell3, kCellThreads), kCellThreads, 0, h->stream>>>(a);
+    launch_after(h, k_list_assign, div_up(h->ngroup, kCellThreads), kCellThreads, 0, a);
+    launch_after(h, k_list_sort, div_up(h->ncell3, kCellThreads), kCellThreads, 0, a);
     h->launches += 2;
   }
   return cudaGetLastError();

@@ -125,6 +125,7 @@ __device__ __forceinline__ void team_sync(int team, int threads)
 template <bool SCREEN, bool GEXCL, bool VIR>
 __global__ void __launch_bounds__(32 * kP64Warps, 1) k_pair_fp64(PairArgs a)
 {
+  after_previous();
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int next_row[kP64Warps];
   constexpr int kMask = kP64Ring - 1, kBytes = p64_warp_bytes(SCREEN, GEXCL, VIR);
@@ -513,6 +514,7 @@ k_sort_sites(const double *__restrict__ r, const double *__restrict__ q, const d
              double4 *__restrict__ sr, double4 *__restrict__ sp, double4 *__restrict__ anchor,
              unsigned long long *__restrict__ counter, int *__restrict__ flags, RebuildArgs rows)
 {
+  after_previous();
   sort_sites(r, q, sig, eps, rscreen, mask, sorted, group, ngroup, G, sr, sp, anchor, counter, flags);
   build_rows(rows);
 }
@@ -520,9 +522,9 @@ k_sort_sites(const double *__restrict__ r, const double *__restrict__ q, const d
 cudaError_t launch_sort_sites(mmnb_handle *h, const double *d_r)
 {
   const int n = h->ngroup * h->G;
-  k_sort_sites<<<sort_blocks(h, n), 32 * kRowWarps, 0, h->stream>>>(d_r, h->d_q, h->d_sig, h->d_eps, h->d_rscreen, h->d_mask,
-                                                      h->d_sorted, h->d_group, h->ngroup, h->G, h->d_sr, h->d_sp,
-                                                      h->d_sanchor, h->d_wsum + 3, h->d_flags, rebuild_args(h));
+  launch_after(h, k_sort_sites, sort_blocks(h, n), 32 * kRowWarps, 0, d_r, h->d_q, h->d_sig, h->d_eps,
+               h->d_rscreen, h->d_mask, h->d_sorted, h->d_group, h->ngroup, h->G, h->d_sr, h->d_sp, h->d_sanchor,
+               h->d_wsum + 3, h->d_flags, rebuild_args(h));
   h->launches += 1;
   return cudaGetLastError();
 }
@@ -554,7 +556,7 @@ static cudaError_t launch_pair64(mmnb_handle *h, PairArgs &a)
                                 (int) room)) != cudaSuccess)
     return e;
   const int grid = std::min(nsm, div_up((long) h->ngroup * a.split, warps));
-  k_pair_fp64<SCREEN, GEXCL, VIR><<<grid, 32 * warps, smem, h->stream>>>(a);
+  launch_after(h, k_pair_fp64<SCREEN, GEXCL, VIR>, grid, 32 * warps, smem, a);
   h->launches += 1;
   return cudaGetLastError();
 }

@@ -107,6 +107,7 @@ __device__ __forceinline__ long long to_fx(float v) { return __float2ll_rn(v * 4
 template <int G, bool SCREEN, bool GEXCL, bool VIR>
 __global__ void __launch_bounds__(32, 20) k_pair_mixed(MixedArgs a)
 {
+  after_previous();
   constexpr int kMask = kMxQueue - 1, kVals = kNacc + (VIR ? 2 : 1);
   __shared__ float4 qda[kMxQueue];   // anchor displacement and r^2
   __shared__ int qj[kMxQueue], qm[kMxQueue], qs[GEXCL ? kMxQueue : 1];
@@ -813,6 +814,7 @@ __device__ __forceinline__ void water_row_store_shfl(const WaterArgs &a, int si0
 template <int MINB, bool VIR, bool UNI>
 __global__ void __launch_bounds__(kWaterWarps * 32, MINB * 4 / kWaterWarps) k_pair_water(WaterArgs a)
 {
+  after_previous();
   // per warp: ring of anchor displacement (xyz, r^2) and the partner's three
   // packed slots
   __shared__ float4 ring[kWaterWarps][4][kWaterRing];
@@ -895,17 +897,17 @@ cudaError_t launch_rspace_water(mmnb_handle *h)
   const int blocks = div_up(h->ngroup, kWaterWarps);
   const bool uni = h->water_uni;
   if (h->want_virial && uni)
-    k_pair_water<4, true, true><<<blocks, kWaterWarps * 32, 0, h->stream>>>(a);
+    launch_after(h, k_pair_water<4, true, true>, blocks, kWaterWarps * 32, 0, a);
   else if (h->want_virial)
-    k_pair_water<4, true, false><<<blocks, kWaterWarps * 32, 0, h->stream>>>(a);
+    launch_after(h, k_pair_water<4, true, false>, blocks, kWaterWarps * 32, 0, a);
   else if (h->tune.water_minb == 5 && uni)
-    k_pair_water<5, false, true><<<blocks, kWaterWarps * 32, 0, h->stream>>>(a);
+    launch_after(h, k_pair_water<5, false, true>, blocks, kWaterWarps * 32, 0, a);
   else if (h->tune.water_minb == 5)
-    k_pair_water<5, false, false><<<blocks, kWaterWarps * 32, 0, h->stream>>>(a);
+    launch_after(h, k_pair_water<5, false, false>, blocks, kWaterWarps * 32, 0, a);
   else if (uni)
-    k_pair_water<4, false, true><<<blocks, kWaterWarps * 32, 0, h->stream>>>(a);
+    launch_after(h, k_pair_water<4, false, true>, blocks, kWaterWarps * 32, 0, a);
   else
-    k_pair_water<4, false, false><<<blocks, kWaterWarps * 32, 0, h->stream>>>(a);
+    launch_after(h, k_pair_water<4, false, false>, blocks, kWaterWarps * 32, 0, a);
   return cudaGetLastError();
 }
 
@@ -1002,6 +1004,7 @@ k_prep_mixed(const double *__restrict__ r, const double *__restrict__ q, const d
              unsigned long long *__restrict__ wsum, int *__restrict__ flags, float4 *__restrict__ anc32, Box box,
              int ncell, double3 edge, double3 inv_edge, RebuildArgs rows)
 {
+  after_previous();
   prep_mixed(r, q, sig, eps, rscreen, mask, sorted, group, ngroup, G, water, site, par, anchor, wsum, flags, anc32,
              box, ncell, edge, inv_edge);
   build_rows(rows);
@@ -1013,10 +1016,9 @@ cudaError_t launch_prep_mixed(mmnb_handle *h, const double *d_r)
   const int water = h->water && !h->want_fields && h->cfg.include_rspace;
   const double3 edge = make_double3((float) h->cg.lc[0], (float) h->cg.lc[1], (float) h->cg.lc[2]);
   const double3 inv_edge = make_double3(1.0 / edge.x, 1.0 / edge.y, 1.0 / edge.z);
-  k_prep_mixed<<<sort_blocks(h, n), 32 * kRowWarps, 0, h->stream>>>(d_r, h->d_q, h->d_sig, h->d_eps, h->d_rscreen, h->d_mask,
-                                                      h->d_sorted, h->d_group, h->ngroup, h->G, water, h->mx.site,
-                                                      h->mx.par, h->mx.anchor, h->d_wsum, h->d_flags, h->mx.anc32,
-                                                      h->box, h->cg.n, edge, inv_edge, rebuild_args(h));
+  launch_after(h, k_prep_mixed, sort_blocks(h, n), 32 * kRowWarps, 0, d_r, h->d_q, h->d_sig, h->d_eps,
+               h->d_rscreen, h->d_mask, h->d_sorted, h->d_group, h->ngroup, h->G, water, h->mx.site, h->mx.par,
+               h->mx.anchor, h->d_wsum, h->d_flags, h->mx.anc32, h->box, h->cg.n, edge, inv_edge, rebuild_args(h));
   h->launches += 1;
   return cudaGetLastError();
 }
@@ -1030,7 +1032,7 @@ static void launch_mixed_g(mmnb_handle *h, const MixedArgs &a)
             : h->has_rscreen
                 ? (h->any_gexcl ? k_pair_mixed<G, true, true, false> : k_pair_mixed<G, true, false, false>)
                 : (h->any_gexcl ? k_pair_mixed<G, false, true, false> : k_pair_mixed<G, false, false, false>);
-  k<<<h->ngroup, 32, 0, h->stream>>>(a);
+  launch_after(h, k, h->ngroup, 32, 0, a);
 }
 
 cudaError_t launch_rspace_mixed(mmnb_handle *h)

@@ -145,6 +145,7 @@ constexpr int w64_words(bool uni) { return uni ? 5 : 8; }
 template <bool VIR, bool UNI>
 __global__ void __launch_bounds__(kW64Warps * 32, 1) k_pair_water64(Water64Args a)
 {
+  after_previous();
   constexpr int kWords = w64_words(UNI);
   extern __shared__ __align__(16) unsigned char smem[];
   // per warp: ring of (x, y), (z, r^2) of the anchor displacement and the partner's
@@ -386,15 +387,16 @@ k_sort_water64(const double *__restrict__ r, const double *__restrict__ q, const
                int ngroup, double4 *__restrict__ anchor, double2 *__restrict__ rec,
                unsigned long long *__restrict__ counter, int *__restrict__ flags, RebuildArgs rows)
 {
+  after_previous();
   sort_water64(r, q, sig, eps, sorted, group, ngroup, anchor, rec, counter, flags);
   build_rows(rows);
 }
 
 cudaError_t launch_sort_water64(mmnb_handle *h, const double *d_r)
 {
-  k_sort_water64<<<sort_blocks(h, h->ngroup), 32 * kRowWarps, 0, h->stream>>>(
-      d_r, h->d_q, h->d_sig, h->d_eps, h->d_sorted, h->d_group, h->ngroup, h->d_sp, reinterpret_cast<double2 *>(h->d_sr), h->d_wsum + 3,
-      h->d_flags, rebuild_args(h));
+  launch_after(h, k_sort_water64, sort_blocks(h, h->ngroup), 32 * kRowWarps, 0, d_r, h->d_q, h->d_sig,
+               h->d_eps, h->d_sorted, h->d_group, h->ngroup, h->d_sp, reinterpret_cast<double2 *>(h->d_sr),
+               h->d_wsum + 3, h->d_flags, rebuild_args(h));
   h->launches += 1;
   return cudaGetLastError();
 }
@@ -423,8 +425,8 @@ static cudaError_t launch_water64(mmnb_handle *h, Water64Args &a)
   if ((e = cudaFuncSetAttribute(k_pair_water64<VIR, UNI>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin)) !=
       cudaSuccess)
     return e;
-  k_pair_water64<VIR, UNI><<<std::min(nsm, div_up(h->ngroup, warps)), 32 * warps, ring * warps + table * a.copies,
-                             h->stream>>>(a);
+  launch_after(h, k_pair_water64<VIR, UNI>, std::min(nsm, div_up(h->ngroup, warps)), 32 * warps,
+               ring * warps + table * a.copies, a);
   h->launches += 1;
   return cudaGetLastError();
 }

@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(kSiteThreads, L == 1 ? 6 : 1) k_sites(SiteArgs
   const int lane = threadIdx.x & 31, c = lane % L;
   const int i = (int) ((blockIdx.x * kSiteThreads + threadIdx.x) >> 5) * S + lane / L;
   const bool live = lane < S * L && i < a.nsite;
+  cudaTriggerProgrammaticLaunchCompletion();
   // exclusion and 1-4 terms of this lane's partners; FP64 mesh terms join them
   double v[4] = {0, 0, 0, 0}, lf[3] = {0, 0, 0}, elj = 0, vir = 0;
   float v32[4] = {0.f, 0.f, 0.f, 0.f};
