@@ -271,7 +271,8 @@ def run_ours(args):
     nsite = wb.nsite
     mesh_pts = MESH ** 3
     alg = {"p3m_spread": nsite * 125 * 8 + nsite * 32,          # 64-bit reductions + positions, charges
-           "p3m_gather": nsite * 125 * 4 + nsite * (24 + 32),   # potential reads + positions, outputs
+           # potential reads + positions, charges and masks, fixed-point sums, forces
+           "sites": nsite * 125 * 4 + nsite * (24 + 12 + 64 + 24),
            "p3m_fft": 2 * (mesh_pts * 4 + MESH * MESH * (MESH // 2 + 1) * 8)}  # one read + write per transform
     roofline["stage_bandwidth_GBs"] = {k: alg[k] / (stages[k] * 1e-3) / 1e9 for k in alg if stages.get(k)}
     roofline["stage_bytes"] = alg
