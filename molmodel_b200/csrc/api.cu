@@ -449,7 +449,7 @@ int setup_p3m(mmnb_handle *h)
       return s;
     CK(cudaMemset(h->d_mesh_fx, 0, sizeof(unsigned long long) * nr));
     if (c.p3m_ik_differentiate)
-      if ((s = dalloc(h, &h->d_egrid32, 3 * nr)) || (s = dalloc(h, &h->d_egridk32, 3 * nk)))
+      if ((s = dalloc(h, &h->d_egrid32, 3 * nr)) || (s = dalloc(h, &h->d_egridk32, 4 * nk)))
         return s;
     if (!h->d_fft32) {
       CKFFT(cufftPlan3d(&h->plan_r2c32, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_R2C));
@@ -468,7 +468,7 @@ int setup_p3m(mmnb_handle *h)
       CKFFT(cufftSetStream(h->plan_c2r, h->stream));
     }
     if (c.p3m_ik_differentiate)
-      if ((s = dalloc(h, &h->d_egrid, 3 * nr)) || (s = dalloc(h, &h->d_egridk, 3 * nk)))
+      if ((s = dalloc(h, &h->d_egrid, 3 * nr)) || (s = dalloc(h, &h->d_egridk, 4 * nk)))
         return s;
   }
   if (h->eta < 0 && (s = p3m_optimize_eta(h, spacing)))

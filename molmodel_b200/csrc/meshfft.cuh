@@ -11,7 +11,7 @@ struct MeshSolve {
   const void *table;     // mesh_fft_table's, on the device
   const T *green;
   const double *kvec;    // per half-spectrum point, for the field spectra
-  void *spec, *fspec;    // half spectrum; null, or room for three more (ik differentiation)
+  void *spec, *fspec;    // half spectrum; null, or room for four (ik differentiation)
   T *out, *fout;         // potential mesh; the three field meshes
 };
 
