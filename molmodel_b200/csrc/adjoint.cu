@@ -413,6 +413,7 @@ static int grad_p3m_scratch(mmnb_handle *h, P3mScratch &s)
 {
   const size_t nr = (size_t) h->mesh[0] * h->mesh[1] * h->mesh[2];
   const size_t nk = (size_t) h->mesh[0] * h->mesh[1] * (h->mesh[2] / 2 + 1);
+  s.own = h->d_fft64 && !h->cfg.p3m_ik_differentiate;
   if (h->cfg.precision != MMNB_MIXED) {
     s.r2c = h->plan_r2c;
     s.c2r = h->plan_c2r;
@@ -430,19 +431,31 @@ static int grad_p3m_scratch(mmnb_handle *h, P3mScratch &s)
   // ik: three spread meshes and the summed spectrum's mesh
   const int nm = h->cfg.p3m_ik_differentiate ? 4 : 1;
   if (!h->d_gmesh) {
-    cudaError_t e = cudaMalloc(&h->d_gmesh, sizeof(double) * nr * nm);
+    // all of it or nothing: after a failure the next call starts over
+    double *mesh = nullptr;
+    cufftDoubleComplex *spec = nullptr;
+    cufftHandle r2c = 0, c2r = 0;
+    cudaError_t e = cudaMalloc(&mesh, sizeof(double) * nr * nm);
     if (e == cudaSuccess)
-      e = cudaMalloc(&h->d_gmeshk, sizeof(cufftDoubleComplex) * nk * nm);
-    if (e != cudaSuccess) {
-      h->err = std::string("gradient mesh: ") + cudaGetErrorString(e);
+      e = cudaMalloc(&spec, sizeof(cufftDoubleComplex) * nk * nm);
+    bool planned = true;
+    if (e == cudaSuccess && !s.own) {
+      planned = cufftPlan3d(&r2c, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_D2Z) == CUFFT_SUCCESS;
+      if (planned && cufftPlan3d(&c2r, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_Z2D) != CUFFT_SUCCESS) {
+        cufftDestroy(r2c);
+        planned = false;
+      }
+    }
+    if (e != cudaSuccess || !planned) {
+      cudaFree(spec);
+      cudaFree(mesh);
+      h->err = e != cudaSuccess ? std::string("gradient mesh: ") + cudaGetErrorString(e) : "gradient mesh: cuFFT plan";
       return MMNB_ERR_CUDA;
     }
-    const bool own = h->d_fft64 && nm == 1;
-    if (!own && (cufftPlan3d(&h->gplan_r2c, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_D2Z) != CUFFT_SUCCESS ||
-        cufftPlan3d(&h->gplan_c2r, h->mesh[0], h->mesh[1], h->mesh[2], CUFFT_Z2D) != CUFFT_SUCCESS)) {
-      h->err = "gradient mesh: cuFFT plan";
-      return MMNB_ERR_CUDA;
-    }
+    h->d_gmesh = mesh;
+    h->d_gmeshk = spec;
+    h->gplan_r2c = r2c;
+    h->gplan_c2r = c2r;
   }
   s.r2c = h->gplan_r2c;
   s.c2r = h->gplan_c2r;

@@ -330,7 +330,8 @@ cudaError_t launch_p3m_fp64(mmnb_handle *h, const double *d_r);
 struct P3mScratch {
   double *spread = nullptr, *solve = nullptr;
   cufftDoubleComplex *spreadk = nullptr, *solvek = nullptr;
-  cufftHandle r2c = 0, c2r = 0;  // or none: own transforms
+  bool own = false;              // the solve is the own transforms' (no plans)
+  cufftHandle r2c = 0, c2r = 0;
 };
 // d_psi += mesh potential of the dipoles q_j g_j (g: 3 per site), FP64
 cudaError_t launch_p3m_dipole_fp64(mmnb_handle *h, const double *d_r, const double *d_g, const P3mScratch &s,

@@ -396,7 +396,7 @@ static cudaError_t p3m_dipole_p(mmnb_handle *h, const double *d_r, const double 
     return e;
   k_spread_dipole_fp64<P><<<lane_blocks<P>(h->nsite), 128, 0, h->stream>>>(m, d_r, h->d_q, h->d_mask, d_g, ik, nr,
                                                                          s.spread);
-  if (!s.r2c) {
+  if (s.own) {
     e = mesh_solve64(h, s.spread, s.spreadk, nullptr, s.solve, nullptr);
     if (e != cudaSuccess)
       return e;
