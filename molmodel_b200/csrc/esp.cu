@@ -54,7 +54,7 @@ struct EspArgs {
   // cells: n per axis, their edges, how many of them the cutoff reaches across
   int n[3], reach[3], ncell;
   float Lf[3], edge[3], reach2, low2;
-  int *cell, *slot, *ids, *count, *start, *poison;
+  int *cell, *slot, *ids, *count, *start, *far;  // far: set when a site is far away (esp_near)
   float4 *near;    // sorted sites wrapped into the box
   double4 *site;   // sorted sites: position and charge
   double *screen;  // sorted sites: r_screen
@@ -74,18 +74,27 @@ __device__ __forceinline__ double esp_b0(const EspArgs &a, double r2)
   return erfc(a.eta * rm) / rm;
 }
 
-// position wrapped into [0, L) and its cell along one axis; in range whatever
-// the coordinate (a conversion of NaN gives 0 and others saturate)
+// Whether a coordinate is near enough to be wrapped: 2^30 box lengths away the wrapped
+// value is off by 2^-22 of one, within the margin of `reach`.  A point or a site
+// farther out (or not finite) has no cell that means anything, and what the minimum
+// image makes of it is rounding: such a point, and every point when a site is such,
+// takes all sites one by one.
+__device__ __forceinline__ bool esp_near(const EspArgs &a, double x, double y, double z)
+{
+  const double m = 1073741824.0;
+  return fabs(x * a.box.invL[0]) <= m && fabs(y * a.box.invL[1]) <= m && fabs(z * a.box.invL[2]) <= m;
+}
+
+// position wrapped into [0, L] and its cell along one axis, both in range whatever the
+// coordinate (a conversion of NaN gives 0 and others saturate), right for a near one
 __device__ __forceinline__ int esp_cell(const EspArgs &a, int d, double x, float &w)
 {
   const double f = x - a.box.L[d] * floor(x * a.box.invL[d]);
-  w = (float) f;
+  w = fminf(fmaxf((float) f, 0.f), a.Lf[d]);
   return min(max((int) (f * a.box.invL[d] * a.n[d]), 0), a.n[d] - 1);
 }
 
-// cell of each site that acts on points, its place there in order of arrival;
-// a coordinate that is not finite poisons every potential, as it would in a
-// sum over all pairs
+// cell of each site that acts on points, its place there in order of arrival
 __global__ void __launch_bounds__(kEspThreads) k_esp_count(EspArgs a)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -96,8 +105,8 @@ __global__ void __launch_bounds__(kEspThreads) k_esp_count(EspArgs a)
     float w;
     const double x = a.r[3 * i], y = a.r[3 * i + 1], z = a.r[3 * i + 2];
     c = (esp_cell(a, 0, x, w) * a.n[1] + esp_cell(a, 1, y, w)) * a.n[2] + esp_cell(a, 2, z, w);
-    if (!isfinite(x) || !isfinite(y) || !isfinite(z))
-      *a.poison = 1;
+    if (!esp_near(a, x, y, z))
+      *a.far = 1;
     a.slot[i] = atomicAdd(a.count + c, 1);
   }
   a.cell[i] = c;
@@ -181,9 +190,6 @@ __global__ void __launch_bounds__(kEspThreads) k_esp_rspace(EspArgs a)
   // take erfc (a handful a point: together, not one or two lanes of every batch)
   int(*const wq)[64] = queue[w];
   const double gx = a.pts[3 * (size_t) j], gy = a.pts[3 * (size_t) j + 1], gz = a.pts[3 * (size_t) j + 2];
-  float px, py, pz;
-  const int cx = esp_cell(a, 0, gx, px), cy = esp_cell(a, 1, gy, py);
-  esp_cell(a, 2, gz, pz);
   double p = 0;
   auto eval = [&](int k) {
     const double4 s = a.site[k];
@@ -205,6 +211,22 @@ __global__ void __launch_bounds__(kEspThreads) k_esp_rspace(EspArgs a)
     }
     p += s.w * b0;
   };
+  auto done = [&]() {
+    for (int o = 16; o > 0; o >>= 1)
+      p += __shfl_xor_sync(0xffffffffu, p, o);
+    if (lane == 0)
+      a.phi[j] = p;
+  };
+  if (*a.far || !esp_near(a, gx, gy, gz)) {
+    for (int k = lane; k < a.start[a.ncell]; k += 32)
+      eval(k);
+    __syncwarp();
+    done();
+    return;
+  }
+  float px, py, pz;
+  const int cx = esp_cell(a, 0, gx, px), cy = esp_cell(a, 1, gy, py);
+  esp_cell(a, 2, gz, pz);
   int qn[2] = {0, 0};
   const int nx = a.n[0], ny = a.n[1], nz = a.n[2];
   const int sx = min(2 * a.reach[0] + 1, nx), sy = min(2 * a.reach[1] + 1, ny);
@@ -296,13 +318,8 @@ __global__ void __launch_bounds__(kEspThreads) k_esp_rspace(EspArgs a)
   for (int g = 0; g < 2; g++)
     if (lane < qn[g])
       eval(wq[g][lane]);
-  for (int o = 16; o > 0; o >>= 1)
-    p += __shfl_xor_sync(0xffffffffu, p, o);
-  if (lane == 0) {
-    if (*a.poison || (a.start[a.ncell] > 0 && !isfinite(gx + gy + gz)))
-      p = NAN;
-    a.phi[j] = p;
-  }
+  __syncwarp();
+  done();
 }
 
 }  // namespace mmnb
@@ -400,8 +417,8 @@ extern "C" int mmnb_phi_at_points(mmnb_handle *h, const double *r, int npoint, c
   a.slot = a.cell + n;
   a.ids = a.slot + n;
   a.count = a.ids + n;  // the counts and the flag behind them are cleared together
-  a.poison = a.count + a.ncell;
-  a.start = a.poison + 1;
+  a.far = a.count + a.ncell;
+  a.start = a.far + 1;
   e = cudaMemcpyAsync(d_r, r, 3 * n * sizeof(double), cudaMemcpyHostToDevice, h->stream);
   if (e == cudaSuccess && c.include_rspace) {
     e = cudaMemsetAsync(a.count, 0, ((size_t) a.ncell + 1) * sizeof(int), h->stream);
