@@ -20,7 +20,11 @@ def check(wb, r, pts):
     o = port().eleclj(make_config(wb.box, **CFG), wb.nsite, wb.groups, wb.exclusions, wb.site_mask, wb.q, wb.sigma,
                       wb.epsilon, np.zeros(wb.nsite))
     phi = ElecLJ(**CFG).init(wb).electrostatic_potential_at_gridpoints(r, pts)
-    assert rel_max(phi, o.phi_at_points(r, pts)) < 1e-10
+    ref = o.phi_at_points(r, pts)
+    # (a displacement rounded to zero gives infinity in either)
+    some = np.isfinite(ref)
+    assert np.array_equal(phi[~some], ref[~some])
+    assert not some.any() or rel_max(phi[some], ref[some]) < 1e-10
 
 
 def box_multiples(box):
