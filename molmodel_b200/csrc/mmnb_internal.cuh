@@ -14,6 +14,7 @@ namespace mmnb {
 constexpr int kCheb = 512;          // Chebyshev segments (include/cheby.h:10)
 constexpr int kChebWMax = 2048;     // segments of the rigid-water FP64 kernel's continued table
 constexpr int kMaxGroup = 8;        // sites per group handled by the pair kernels
+constexpr int kTailMax = 512;       // segments of the general kernel's continuation
 constexpr int kMaxOrder = 7;        // P3M assignment order (src/pppm.c:61)
 constexpr int kWarp = 32;
 
@@ -142,9 +143,11 @@ struct mmnb_handle {
   int *d_mask = nullptr;
   double *d_q = nullptr, *d_sig = nullptr, *d_eps = nullptr, *d_rscreen = nullptr;
   double cheb_min = 0, cheb_max = 0, cheb_inv_dx = 0;
-  // the rigid-water FP64 kernel's table: cheb_w_nseg x (c0, c1), then x (c2, c3)
+  // the rigid-water FP64 kernel's table: cheb_w_nseg x (c0, c1), then x (c2, c3); then
+  // the general one's continuation from cheb_max on, tail_nseg x 8 coefficients
   double *d_cheb_w = nullptr;
-  int cheb_w_nseg = 0;
+  int cheb_w_nseg = 0, tail_nseg = 0;
+  double tail_inv = 0;               // 1 / width of a tail segment
   // 512 x 4: the cubics of -eta d/d(eta) of the table (mmnb_virial)
   double *d_cheb_d = nullptr;
 
@@ -449,11 +452,12 @@ __device__ __forceinline__ double anchor_disp(const Box &b, double4 ri, double4 
 
 #endif
 
-// Segments of the continued table the FP64 pair kernels use.  Past 1.2 rc^2 the
-// reference evaluates erfc and exp; the cubics continued there are within ~1e-9 of
-// those, relatively, which is below 1e-12 of the pair's terms once erfc(eta r) has
-// fallen below ~4e-4 (eta rc >= 2.3, as any screening that makes the cutoff worth
-// anything has it).  Below that the kernels, too, take the exact functions.
+// Segments of the continued table the rigid-water FP64 kernel uses.  Past 1.2 rc^2 the
+// reference evaluates erfc and exp; the cubics continued there are within 1.1e-10 of
+// them for b0 and 1.3e-7 for b1, relatively (rc 9, eta 0.35; 3e-8 for b1 at eta rc =
+// 2.3), in b1 an absolute 4e-15 to 8e-13 where the table itself, inside its range, is
+// off by up to 1.5e-6.  From eta rc = 2.3 on, where erfc(eta r) has fallen below ~4e-4,
+// that is below 1e-12 of the pair's terms; under it the exact functions are taken.
 inline double table_segments(const mmnb_handle *h)
 {
   return h->eta * h->rc >= 2.3 ? h->cheb_w_nseg : kCheb;

@@ -31,11 +31,14 @@
 //     partners' sites per step for n row sites.  No lane holds a site that lacks
 //     the term, so the sums of a lane are one site's: 12 doubles at most, and the
 //     kernel is the same for groups of one site and of eight.
-// The reference's table (continued past 1.2 rc^2 by segments of the same
-// construction where table_segments allows it) is in shared memory, the cubic
-// alone: b1 is -2 / dx times its derivative, which is how the reference stores it;
-// below the table (r^2 < 4) ewald_short.  Lanes' sums are added in a fixed order:
-// no atomics, bitwise reproducible whichever warp takes a row.
+// The reference's table is in shared memory, the cubic alone: b1 is -2 / dx times its
+// derivative, which is how the reference stores it; below the table (r^2 < 4)
+// ewald_short, past it (r^2 > 1.2 rc^2) polynomials of degree seven that are the
+// function to rounding, where the reference takes erfc and exp (which a few lanes of
+// nearly every step would take, the others waiting: 17^3 cells of solution, per call,
+// 134 us with the functions, 127 with these).
+// Lanes' sums are added in a fixed order: no atomics, bitwise reproducible whichever
+// warp takes a row.
 //
 // Bound by latency (12 warps of 168 registers per SM; 16 of 128 spill and were
 // slower, 86 against 115 us) and the shared-memory pipe.  Measured on 17^3 cells of
@@ -57,11 +60,13 @@ constexpr int kP64Warps = 12;  // at most, per block: 168 registers a thread, no
 constexpr int kP64Ring = 64;   // entries per queue: at most 31 carried over and 32 new
 
 struct PairArgs {
-  int ngroup, rowcap, geometric, G, width, batch, split, nseg, copies, series;
+  int ngroup, rowcap, geometric, G, width, batch, split, copies, series, half;  // half: entries to the (c2, c3)
   Box box;
   double rlo2, rhi2, inv_sw, eta, eta2, cerf;  // cerf = 2 eta / sqrt(pi)
-  double cmin, inv_dx, dscale, inv_dscale, nsegd;  // dscale = -2 / segment width
-  const double2 *table;                        // [nseg] (c0, c1), then [nseg] (c2, c3)
+  double cmin, inv_dx, dscale, inv_dscale;     // dscale = -2 / segment width
+  const double2 *table;                        // (c0, c1) of each segment, from `half` on (c2, c3)
+  const double2 *tail;                         // past the table: 4 per segment, powers 0..7 of its position
+  double tmin, tail_inv, tail_nseg, tscale;    // tscale: b1 / dscale from the position's derivative
   const double4 *anchor;  // sorted groups: anchor, packed first site and site masks
   const double4 *sr;      // slots: offset from the anchor, charge
   const double4 *sp;      // slots: sig, sqrt(eps), rscreen, -
@@ -85,7 +90,7 @@ __device__ __forceinline__ void ewald_p64(const PairArgs &a, const double2 *t0, 
                                           double &b0, double &g, int &seg, double &f)
 {
   const double x = (r2 - a.cmin) * a.inv_dx;
-  if (x > 0 && x < a.nsegd) {
+  if (x > 0 && x < kCheb) {
     // floor(x) exactly: x + 2^52 rounded down holds floor(x) in its low word
     const double t = __dadd_rd(x, 4503599627370496.0);
     const int i = __double2loint(t);
@@ -98,9 +103,24 @@ __device__ __forceinline__ void ewald_p64(const PairArgs &a, const double2 *t0, 
   }
   seg = -1;
   f = 0;
+  const double y = (r2 - a.tmin) * a.tail_inv;
   if (x <= 0 && a.series) {
     ewald_short(a.eta2, a.cerf, r2, b0, g);
     g *= a.inv_dscale;
+  } else if (x > 0 && y < a.tail_nseg) {
+    const int i = (int) y;
+    const double u = fma(2.0, y - i, -1.0);
+    const double2 *const c = a.tail + 4 * i;
+    const double2 c01 = __ldg(c), c23 = __ldg(c + 1), c45 = __ldg(c + 2), c67 = __ldg(c + 3);
+    const double k[8] = {c01.x, c01.y, c23.x, c23.y, c45.x, c45.y, c67.x, c67.y};
+    double p = k[7], d = 0;
+#pragma unroll
+    for (int n = 6; n >= 0; n--) {
+      d = fma(d, u, p);
+      p = fma(p, u, k[n]);
+    }
+    b0 = p;
+    g = d * a.tscale;
   } else {
     const double r = sqrt(r2);
     const double er = a.eta * r;
@@ -130,12 +150,14 @@ __global__ void __launch_bounds__(32 * kP64Warps, 1) k_pair_fp64(PairArgs a)
   __shared__ int next_row[kP64Warps];
   constexpr int kMask = kP64Ring - 1, kBytes = p64_warp_bytes(SCREEN, GEXCL, VIR);
   double2 *const tab = reinterpret_cast<double2 *>(smem);
-  for (int i = threadIdx.x; i < 2 * a.nseg * a.copies; i += blockDim.x)
-    tab[i] = a.table[i / a.copies];
+  for (int i = threadIdx.x; i < 2 * kCheb * a.copies; i += blockDim.x) {
+    const int k = i / a.copies;
+    tab[i] = a.table[k < kCheb ? k : a.half + k - kCheb];
+  }
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   // this lane's copy of the table
-  const double2 *const t0 = tab + lane % a.copies, *const t1 = t0 + a.nseg * a.copies;
-  unsigned char *const base_w = smem + sizeof(double2) * 2 * a.nseg * a.copies;
+  const double2 *const t0 = tab + lane % a.copies, *const t1 = t0 + kCheb * a.copies;
+  unsigned char *const base_w = smem + sizeof(double2) * 2 * kCheb * a.copies;
   auto queues = [&](int warp) { return reinterpret_cast<double2 *>(base_w + (size_t) warp * kBytes); };
   // queued partners: (x, y), (z, r^2) of the anchor displacement
   double2 *const ga = queues(w), *const gb = ga + kP64Ring;
@@ -305,7 +327,7 @@ __global__ void __launch_bounds__(32 * kP64Warps, 1) k_pair_fp64(PairArgs a)
           double b0, g, f;
           int seg;
           ewald_p64(a, t0, t1, r2, b0, g, seg, f);
-          if (VIR && seg >= 0 && seg < kCheb) {
+          if (VIR && seg >= 0) {
             // the table is refitted for each eta: its eta derivative along the
             // volume-move path is the fitted cubic, not b1 r^2 - b0, the identity
             // of the exact function that mmnb_virial's scale covariance assumes
@@ -544,7 +566,7 @@ static cudaError_t launch_pair64(mmnb_handle *h, PairArgs &a)
   a.split = h->ngroup * 4L <= chip ? 4 : h->ngroup * 2L <= chip ? 2 : 1;
   int warps = std::min(kP64Warps, (div_up((long) h->ngroup * a.split, nsm) + 3) / 4 * 4);
   const int per = p64_warp_bytes(SCREEN, GEXCL, VIR);
-  const size_t table = sizeof(double2) * 2 * (size_t) h->cheb_w_nseg, room = (size_t) optin - 1024;
+  const size_t table = sizeof(double2) * 2 * kCheb, room = (size_t) optin - 1024;
   while (warps > 4 && table + (size_t) warps * per > room)
     warps -= 4;
   // a second copy of the table, interleaved so that two lanes of a 16-byte access
@@ -570,7 +592,12 @@ cudaError_t launch_rspace_fp64(mmnb_handle *h)
   a.G = h->G;
   a.width = h->maxgs;
   a.batch = 32 / h->maxgs;
-  a.nseg = h->cheb_w_nseg;
+  a.half = h->cheb_w_nseg;
+  a.tail = reinterpret_cast<const double2 *>(h->d_cheb_w) + 2 * h->cheb_w_nseg;
+  a.tmin = h->cheb_max;
+  a.tail_inv = h->tail_inv;
+  a.tail_nseg = h->tail_nseg;
+  a.tscale = 2 * h->tail_inv * (-2.0) / (-2 * h->cheb_inv_dx);
   a.series = h->eta * sqrt(h->cheb_min) <= kErfSeriesMax;
   a.box = h->box;
   a.rlo2 = h->rlo2;
@@ -583,7 +610,6 @@ cudaError_t launch_rspace_fp64(mmnb_handle *h)
   a.inv_dx = h->cheb_inv_dx;
   a.dscale = -2 * h->cheb_inv_dx;
   a.inv_dscale = 1.0 / a.dscale;
-  a.nsegd = table_segments(h);
   a.table = reinterpret_cast<const double2 *>(h->d_cheb_w);
   a.anchor = h->d_sanchor;
   a.sr = h->d_sr;
