@@ -290,7 +290,7 @@ int setup_cells(mmnb_handle *h)
   }
   if ((s = upload(h, &h->d_cell_rank, rank)) || (s = upload(h, &h->d_cell_of_rank, of_rank)))
     return s;
-  if ((s = dalloc(h, &h->d_cell_count, h->ncell3)) || (s = dalloc(h, &h->d_cell_start, h->ncell3 + 1)) ||
+  if ((s = dalloc(h, &h->d_cell_count, cell_words(h->ncell3))) || (s = dalloc(h, &h->d_cell_start, h->ncell3 + 1)) ||
       (s = dalloc(h, &h->d_cell_head, h->ncell3)))
     return s;
   h->first = true;

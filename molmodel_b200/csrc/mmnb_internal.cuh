@@ -159,7 +159,7 @@ struct mmnb_handle {
   int *d_cell_rank = nullptr;        // reference cell index -> Morton rank
   int *d_cell_of_rank = nullptr;     // Morton rank -> reference cell index
   int *d_cell_of_group = nullptr;    // per group, reference numbering
-  int *d_cell_count = nullptr;       // per rank
+  int *d_cell_count = nullptr;       // per rank, then per chunk of ranks (cell_words)
   int *d_cell_start = nullptr;       // per rank, ncell3+1
   int *d_cell_head = nullptr;        // per rank, the cell's last group to arrive
   int *d_slot = nullptr;             // per group, the group that arrived in its cell before
@@ -464,6 +464,19 @@ inline double table_segments(const mmnb_handle *h)
 }
 
 inline int div_up(long a, long b) { return (int) ((a + b - 1) / b); }
+
+// The list's cells in chunks of 2^chunk_shift, at most kMaxChunks of them: the counts
+// of the cells, padded to whole 16-byte words, then those of the chunks
+constexpr int kMaxChunks = 4096;
+inline int chunk_shift(int ncell3)
+{
+  int s = 6;
+  while (div_up(ncell3, 1 << s) > kMaxChunks)
+    s++;
+  return s;
+}
+inline int chunk_at(int ncell3) { return div_up(ncell3, 4) * 4; }
+inline int cell_words(int ncell3) { return chunk_at(ncell3) + div_up(ncell3, 1 << chunk_shift(ncell3)); }
 
 #ifdef __CUDACC__
 // A kernel behind another one in the handle's stream: on a box small enough its blocks

@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(kCheckThreads) k_list_check(const double *__re
                                                               int first, int force, int interval,
                                                               double *__restrict__ anchor,
                                                               double *__restrict__ partial, int *__restrict__ flags,
-                                                              int *__restrict__ cell_count, int ncell3,
+                                                              int *__restrict__ cell_count, int ncount,
                                                               double prune, const int *__restrict__ rank,
                                                               const double *__restrict__ plast)
 {
@@ -164,15 +164,16 @@ __global__ void __launch_bounds__(kCheckThreads) k_list_check(const double *__re
   }
   __syncthreads();
   if (rebuild_s)
-    for (int c = threadIdx.x; c < ncell3; c += blockDim.x)
+    for (int c = threadIdx.x; c < ncount; c += blockDim.x)
       cell_count[c] = 0;
 }
 
 constexpr int kCellThreads = 256;       // blocks of the two-kernel cell sort
 constexpr int kOneBlockThreads = 1024;  // the one-block cell sort
 
-// cell = round(x / l_cell) mod n per axis; the anchors become the new "last"
-__device__ __forceinline__ void cell_assign(const RebuildArgs &a, int g)
+// Morton rank of group g's cell = round(x / l_cell) mod n per axis; the anchors become
+// the new "last"
+__device__ __forceinline__ int cell_assign(const RebuildArgs &a, int g)
 {
   const int n = a.cg.n;
   int ijk[3];
@@ -190,9 +191,7 @@ __device__ __forceinline__ void cell_assign(const RebuildArgs &a, int g)
   }
   const int c = (ijk[0] * n + ijk[1]) * n + ijk[2];
   a.cell_of_group[g] = c;
-  const int k = a.cell_rank[c];
-  atomicAdd(a.cell_count + k, 1);
-  a.next[g] = atomicExch(a.head + k, g);
+  return a.cell_rank[c];
 }
 
 // Exclusive scan of the values of a block of T threads (one per thread): the
@@ -237,125 +236,171 @@ __device__ __forceinline__ void place_group(const RebuildArgs &a, int g, int pos
   a.anchor32[pos] = make_float4(w[0], w[1], w[2], 0.f);
 }
 
-// The cells of ranks [c0, c0 + T), a thread each: offsets from `base` on (the groups
-// of the cells before), and the cells' groups in index order (deterministic lists).
-// A cell's groups hang on a list in order of arrival; a few are ordered by walking
-// it once per group, the groups of a crowded cell by the whole block.  Returns the
-// offset after the last cell.
-constexpr int kCrowd = 16;
-
-template <int T>
-__device__ int sort_cells(const RebuildArgs &a, int c0, int base, int *warp_tot)
+// groups of the cells before cell k: those of the chunks before its own (`before`, in
+// shared memory) and of the cells before it there
+__device__ __forceinline__ int cell_offset(const RebuildArgs &a, const int *before, int k)
 {
-  __shared__ int crowd[T], ncrowd;
-  if (threadIdx.x == 0)
-    ncrowd = 0;
-  const int c = c0 + threadIdx.x;
-  const int n = c < a.ncell3 ? __ldcg(a.cell_count + c) : 0;
-  int total;
-  const int at = base + block_exclusive_scan<T>(n, warp_tot, total);
-  if (c < a.ncell3)
-    a.start[c] = at;
-  if (c == a.ncell3 - 1)
-    a.start[a.ncell3] = at + n;
-  const int head = n > 0 ? __ldcg(a.head + c) : 0;
-  if (n == 1) {
-    place_group(a, head, at);
-  } else if (n > kCrowd) {
-    int g = head;
-    for (int k = 0; k < n; k++, g = __ldcg(a.next + g))
-      a.scatter[at + k] = g;
-    crowd[atomicAdd(&ncrowd, 1)] = threadIdx.x;
-  } else if (n > 1) {
-    int m[kCrowd];
-    int g = head;
-#pragma unroll
-    for (int k = 0; k < kCrowd; k++) {
-      m[k] = 0x7fffffff;
-      if (k < n) {
-        m[k] = g;
-        if (k + 1 < n)
-          g = __ldcg(a.next + g);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < kCrowd; k++) {
-      if (k >= n)
-        break;
-      int r = 0;
-#pragma unroll
-      for (int j = 0; j < kCrowd; j++)
-        r += m[j] < m[k];
-      place_group(a, m[k], at + r);
-    }
+  const int c = k >> a.chunk_shift;
+  int v = before[c];
+#pragma unroll 4
+  for (int i = c << a.chunk_shift; i < k; i += 4) {
+    const int4 n = __ldcg(reinterpret_cast<const int4 *>(a.cell_count + i));
+    v += n.x + (i + 1 < k ? n.y : 0) + (i + 2 < k ? n.z : 0) + (i + 3 < k ? n.w : 0);
   }
-  __syncthreads();
-  for (int q = 0; q < ncrowd; q++) {
-    const int cq = c0 + crowd[q], b = a.start[cq], e = b + __ldcg(a.cell_count + cq);
-    for (int i = b + threadIdx.x; i < e; i += T) {
-      const int g = a.scatter[i];
-      int r = 0;
-      for (int j = b; j < e; j++)
-        r += a.scatter[j] < g;
-      place_group(a, g, b + r);
-    }
-  }
-  __syncthreads();
-  return base + total;
+  return v;
 }
 
 // Cells and sorted order of a rebuild.  Without one due every block returns at once
 // (the decision is read from device memory, so the launches sit in a CUDA graph
 // unchanged).  As phases of one cooperative launch with the rows, separated by grid
-// barriers, they cost every evaluation a wait for the whole grid's room: the 648-site
-// k-sum box 90 -> 80 us per call, twelve replicas at once 3700 -> 3410 us per ten
-// steps, 98,304 sites mixed 186 -> 178 us.
+// barriers, they cost every evaluation a wait for the whole grid's room (together with
+// the site kernel's change: the 648-site k-sum box 90 -> 86 us per call, twelve
+// replicas at once 3432 -> 3373 us per ten steps, 98,304 sites mixed 177 -> 175.5 us).
 __global__ void __launch_bounds__(kCellThreads) k_list_assign(RebuildArgs a)
 {
   after_previous();
   if (!a.flags[kFlagRebuild])
     return;
   const int g = blockIdx.x * kCellThreads + threadIdx.x;
-  if (g < a.ngroup)
-    cell_assign(a, g);
+  if (g >= a.ngroup)
+    return;
+  const int k = cell_assign(a, g);
+  a.rank_of_group[g] = k;
+  atomicAdd(a.cell_count + k, 1);
+  atomicAdd(a.chunk + (k >> a.chunk_shift), 1);
+  a.next[g] = atomicExch(a.head + k, g);
 }
+
+// Offsets of the cells, a thread each; then a thread per group, its place among its
+// cell's groups in index order (deterministic lists).  A cell's groups hang on a list in
+// order of arrival, and each walks it to count those before it: two on average, tens
+// in a droplet or a cluster, whose few cells a thread per cell would leave to a few
+// threads (32,768 waters as a droplet in 20 times the volume, mixed, list rebuilt in
+// each call: 573 us so, 297 now; 302 with a cooperative launch for all phases).
+// Past kWalk of them (all coordinates zero, or not finite) a block counts the cell's
+// groups of the blocks before instead, in order.
+constexpr int kWalk = 512;
 
 __global__ void __launch_bounds__(kCellThreads) k_list_sort(RebuildArgs a)
 {
+  constexpr int T = kCellThreads;
   after_previous();
   if (!a.flags[kFlagRebuild])
     return;
-  __shared__ int warp_tot[kCellThreads / 32];
-  // groups of the blocks before
-  const int c0 = blockIdx.x * kCellThreads;
-  int v = 0, base;
-#pragma unroll 8
-  for (int i = threadIdx.x; i < c0; i += kCellThreads)
-    v += __ldcg(a.cell_count + i);
-  block_exclusive_scan<kCellThreads>(v, warp_tot, base);
-  sort_cells<kCellThreads>(a, c0, base, warp_tot);
+  extern __shared__ int before[];  // nchunk
+  __shared__ int warp_tot[T / 32], pick;
+  int total, run = 0;
+  for (int c0 = 0; c0 < a.nchunk; c0 += T) {
+    const int c = c0 + threadIdx.x;
+    const int ex = block_exclusive_scan<T>(c < a.nchunk ? a.chunk[c] : 0, warp_tot, total);
+    if (c < a.nchunk)
+      before[c] = run + ex;
+    run += total;
+  }
+  __syncthreads();
+  const int g0 = blockIdx.x * T, g = g0 + threadIdx.x;
+  if (g < a.ncell3) {
+    a.start[g] = cell_offset(a, before, g);
+    if (g == a.ncell3 - 1)
+      a.start[a.ncell3] = a.ngroup;
+  }
+  int k = 0, n = 0, at = 0;
+  if (g < a.ngroup) {
+    k = a.rank_of_group[g];
+    n = a.cell_count[k];
+    int h = a.head[k];
+    at = cell_offset(a, before, k);
+    if (n <= kWalk) {
+      for (int i = 1; i < n; i++) {
+        at += h < g;
+        h = a.next[h];
+      }
+      at += h < g;
+      place_group(a, g, at);
+    }
+  }
+  bool crowd = n > kWalk;
+  while (__syncthreads_or(crowd)) {
+    if (threadIdx.x == 0)
+      pick = a.ncell3;
+    __syncthreads();
+    if (crowd)
+      atomicMin(&pick, k);
+    __syncthreads();
+    const int cell = pick;
+    int v = 0;
+    for (int j = threadIdx.x; j < g0; j += T)
+      v += a.rank_of_group[j] == cell;
+    int earlier;
+    block_exclusive_scan<T>(v, warp_tot, earlier);
+    const bool in = crowd && k == cell;
+    const int ex = block_exclusive_scan<T>(in ? 1 : 0, warp_tot, total);
+    if (in) {
+      place_group(a, g, at + earlier + ex);
+      crowd = false;
+    }
+  }
 }
 
-// both steps by one block, for boxes it handles as fast as two launches would
+// The same by one block, for boxes it handles as fast as two launches would: counts and
+// order in shared memory, the groups ordered by comparing all of their cell's.
+constexpr int kOneBlockGroups = 2048, kOneBlockCells = 1024;
+constexpr int kOneBlockEach = kOneBlockGroups / kOneBlockThreads;
+
 __global__ void __launch_bounds__(kOneBlockThreads) k_list_cells(RebuildArgs a)
 {
+  static_assert(kOneBlockCells <= kOneBlockThreads, "a cell per thread");
   after_previous();
   if (!a.flags[kFlagRebuild])
     return;
-  __shared__ int warp_tot[kOneBlockThreads / 32];
-  for (int g = threadIdx.x; g < a.ngroup; g += kOneBlockThreads)
-    cell_assign(a, g);
+  __shared__ int count[kOneBlockCells], start[kOneBlockCells], list[kOneBlockGroups], warp_tot[kOneBlockThreads / 32];
+  const int t = threadIdx.x;
+  if (t < kOneBlockCells)
+    count[t] = 0;
   __syncthreads();
-  int base = 0;
-  for (int c0 = 0; c0 < a.ncell3; c0 += kOneBlockThreads)
-    base = sort_cells<kOneBlockThreads>(a, c0, base, warp_tot);
+  int k[kOneBlockEach], slot[kOneBlockEach];
+#pragma unroll
+  for (int i = 0; i < kOneBlockEach; i++) {
+    const int g = t + i * kOneBlockThreads;
+    if (g < a.ngroup) {
+      k[i] = cell_assign(a, g);
+      slot[i] = atomicAdd(count + k[i], 1);
+    }
+  }
+  __syncthreads();
+  int total;
+  const int at = block_exclusive_scan<kOneBlockThreads>(t < a.ncell3 ? count[t] : 0, warp_tot, total);
+  if (t < a.ncell3)
+    start[t] = a.start[t] = at;
+  if (t == 0)
+    a.start[a.ncell3] = a.ngroup;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kOneBlockEach; i++) {
+    const int g = t + i * kOneBlockThreads;
+    if (g < a.ngroup)
+      list[start[k[i]] + slot[i]] = g;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kOneBlockEach; i++) {
+    const int g = t + i * kOneBlockThreads;
+    if (g < a.ngroup) {
+      const int b = start[k[i]], n = count[k[i]];
+      int r = 0;
+#pragma unroll 4
+      for (int j = 0; j < n; j++)
+        r += list[b + j] < g;
+      place_group(a, g, b + r);
+    }
+  }
 }
 
 cudaError_t launch_list_check(mmnb_handle *h, const double *d_r, int force)
 {
   k_list_check<<<h->top2_blocks, kCheckThreads, 0, h->stream>>>(
       d_r, h->d_group, h->ngroup, h->d_last, h->nlw, h->first ? 1 : 0, force, h->cfg.rebuild_interval, h->d_anchor,
-      h->d_top2, h->d_flags, h->d_cell_count, h->ncell3, h->water ? h->prune_margin : 0.0, h->d_rank,
+      h->d_top2, h->d_flags, h->d_cell_count, cell_words(h->ncell3), h->water ? h->prune_margin : 0.0, h->d_rank,
       h->d_plast);
   h->launches += 1;
   return cudaGetLastError();
@@ -387,8 +432,11 @@ RebuildArgs rebuild_args(const mmnb_handle *h)
   a.nbr_count = h->d_nbr_count;
   a.anchor32 = h->d_anchor32;
   // the rows' counts are written last, by the list build: until then they
-  // hold the groups in cell order
-  a.scatter = h->d_nbr_count;
+  // hold the rank of each group's cell
+  a.rank_of_group = h->d_nbr_count;
+  a.chunk_shift = chunk_shift(h->ncell3);
+  a.chunk = h->d_cell_count + chunk_at(h->ncell3);
+  a.nchunk = div_up(h->ncell3, 1 << a.chunk_shift);
   // bound of the FP32 squared-distance error: anchors wrapped into [0, L] and
   // rounded (<= 4 ulp(L) per component after the difference and the image
   // shift), propagated through |d|^2, plus the rounding of the sum; 8x margin
@@ -415,20 +463,21 @@ RebuildArgs rebuild_args(const mmnb_handle *h)
   return a;
 }
 
-// The one-block sort up to this many groups: a launch less in every evaluation
-// (~1.3 us), against a slower rebuild (profiled cold, 512 groups: 9 us in one block;
-// 4,096 groups: 33 us against 5 + 12; 32,768 in one block 147 us against 5 + 15)
-constexpr int kOneBlockGroups = 2048;
-
+// The one-block sort up to kOneBlockGroups (of ncell3 <= ngroup / 2 + 3 cells): a launch
+// less in every evaluation, and a faster rebuild up to about there.  Calls with the list
+// rebuilt in each, one block against two kernels, mixed: 216 waters 38.7 and 42.8 us,
+// 1,000 44.8 and 48.5, 1,500 49.4 and 49.4, 2,048 53.5 and 50.3; rebuilt every ten
+// calls: 27.9 and 29.1, 32.0 and 32.7, 34.4 and 34.7, 36.7 and 36.9.
 cudaError_t launch_list_cells(mmnb_handle *h)
 {
   const RebuildArgs a = rebuild_args(h);
-  if (h->ngroup <= kOneBlockGroups) {
+  if (h->ngroup <= kOneBlockGroups && h->ncell3 <= kOneBlockCells) {
     launch_after(h, k_list_cells, 1, kOneBlockThreads, 0, a);
     h->launches += 1;
   } else {
     launch_after(h, k_list_assign, div_up(h->ngroup, kCellThreads), kCellThreads, 0, a);
-    launch_after(h, k_list_sort, div_up(h->ncell3, kCellThreads), kCellThreads, 0, a);
+    launch_after(h, k_list_sort, div_up(std::max(h->ngroup, h->ncell3), kCellThreads), kCellThreads,
+                 sizeof(int) * a.nchunk, a);
     h->launches += 2;
   }
   return cudaGetLastError();

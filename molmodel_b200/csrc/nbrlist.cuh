@@ -38,7 +38,9 @@ struct RebuildArgs {
   // sqrt(c2cull) > cutoff + width from the row's anchor holds no partner
   float lcf[3], c2cull;
   int *head;                 // per rank: the cell's last group to arrive
-  int *scatter;              // scratch, ngroup: a crowded cell's groups
+  int *rank_of_group;        // scratch, ngroup: the Morton rank of each group's cell
+  int *chunk;                // groups of each 2^chunk_shift cells (ranks)
+  int chunk_shift, nchunk;
 };
 
 // one warp per sorted group.  Per batch of 32 stencil cells the members are
