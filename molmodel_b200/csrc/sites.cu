@@ -22,11 +22,10 @@
 // As three kernels (exclusions, interpolation, assembly) the sites' potential,
 // field and LJ force went through memory between them and each waited for the
 // last (profiled one by one, caches cold): 98,304 sites 32.5 us mixed, 59 us FP64;
-// 12,288 sites 26 and 37 us.  This kernel, a lane per mesh plane: 54 and 80 us, 14
-// and 14 us; a lane per site: 25 and 35 us, 15 and 17 us; with 16 bytes of a mesh row
-// a load 24 and 31 us.  Bound by the loads' latency (10 of a warp's 18 cycles between
-// instructions, one wave of 20 warps an SM): a site's lanes cover it where the sites
-// alone would leave the chip idle, and repeat its weights where they would not.
+// 12,288 sites 26 and 37 us.  This kernel, in a step with stage timing: 98,304 sites 26
+// us mixed, 29 FP64; 12,288 sites 14 and 15.  Bound by the loads' latency: a site's lanes
+// cover it where the sites alone would leave the chip idle, and repeat its weights where
+// they would not.
 
 #include "mesh.cuh"
 
@@ -106,40 +105,28 @@ __device__ __forceinline__ void excluded_b(const SiteArgs &a, double r2, double 
   }
 }
 
-// a mesh row's points of one lane, 16 bytes a load when whole rows allow it
-template <typename T, int V>
-struct MeshVec {
-  T v[V];
-};
-template <int V>
-__device__ __forceinline__ MeshVec<float, V> mesh_load(const float *p)
+// Blocks an SM the register budget is cut for, a lane per site.  The sites' loads want
+// many warps, a spilled order takes more from them than they give, and the best cut
+// moves with the order's arrays.  32,768 waters, the step in us at 6 / 4 / 3 / 2 blocks:
+//   FP64  order 3: 228 / 232 / 233 / 232    mixed  122 / 126 / 124 / -
+//         order 4: 256 / 245 / 244 / 248           133 / 136 / 135 / -
+//         order 5: 285 / 263 / 257 / 262           154 / 147 / 149 / 154
+//         order 6: 324 / 313 / 285 / 284           181 / 169 / 171 / 176
+//         order 7: 383 / 361 / 332 / 316           222 / 209 / 190 / 196
+//   with ik, 5:    372 / 372 / 367 / 368           199 / 207 / 206 / -
+//            7:    521 / 519 / 481 / 470           297 / 293 / 269 / 286
+// (orders 5 and 7 of 66,000 sites with ik, mixed: one wave at 4 blocks, 149 us; 154 at
+// 6, 163 at 3.)  One cap of 6 for all, which order 5's whole-word rows were measured
+// with, spilled up to 6 KB a thread: order 7 388 us FP64 and 233 mixed on rows of 81.
+constexpr int site_blocks_per_sm(int P, MeshKind kind)
 {
-  MeshVec<float, V> o;
-  if constexpr (V == 4) {
-    const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
-    o.v[0] = t.x, o.v[1] = t.y, o.v[2] = t.z, o.v[3] = t.w;
-  } else {
-    o.v[0] = __ldg(p);
-  }
-  return o;
-}
-template <int V>
-__device__ __forceinline__ MeshVec<double, V> mesh_load(const double *p)
-{
-  MeshVec<double, V> o;
-  if constexpr (V == 2) {
-    const double2 t = __ldg(reinterpret_cast<const double2 *>(p));
-    o.v[0] = t.x, o.v[1] = t.y;
-  } else {
-    o.v[0] = __ldg(p);
-  }
-  return o;
+  const bool k32 = kind == kMesh32 || kind == kMesh32Ik, ik = kind == kMesh64Ik || kind == kMesh32Ik;
+  return P <= 3 || (k32 && P == 4) ? 6 : P == 4 || (k32 && P == 5) ? 4 : !k32 && (P == 7 || ik) ? 2 : 3;
 }
 
-// P: assignment order, or 0 without a mesh; L: lanes per site (P or one with a mesh);
-// V: mesh points per load (one lane per site and rows of whole 16-byte words; else 1)
-template <int P, MeshKind KIND, int L, int V>
-__global__ void __launch_bounds__(kSiteThreads, L == 1 ? 6 : 1) k_sites(SiteArgs a)
+// P: assignment order, or 0 without a mesh; L: lanes per site (P or one with a mesh)
+template <int P, MeshKind KIND, int L>
+__global__ void __launch_bounds__(kSiteThreads, L == 1 ? site_blocks_per_sm(P, KIND) : 1) k_sites(SiteArgs a)
 {
   constexpr int S = 32 / L;
   constexpr bool k32 = KIND == kMesh32 || KIND == kMesh32Ik, kIk = KIND == kMesh64Ik || KIND == kMesh32Ik;
@@ -167,42 +154,10 @@ __global__ void __launch_bounds__(kSiteThreads, L == 1 ? 6 : 1) k_sites(SiteArgs
     if constexpr (KIND != kNoMesh) {
       typedef typename std::conditional<k32, float, double>::type T;
       constexpr int NZ = L == 1 ? P : 1;  // points along z of this lane
-      constexpr int NV = V == 1 ? NZ : (V - 1 + P + V - 1) / V;  // loads a row
       MeshRows<P, NZ, T> o;
       mesh_rows<P, NZ, T>(a.mesh, a.r + 3 * (size_t) i, c, o);
       const T *const mesh = k32 ? (const T *) a.mesh32 : (const T *) a.mesh64;
       const T *const eg = k32 ? (const T *) a.egrid32 : (const T *) a.egrid64;
-      // the row's words and the weights of their points: with whole words the P points
-      // start at point `sh0` of the first, the others weigh nothing
-      T wz[NV * V], dz[NV * V];
-      int iz[NV];
-      if constexpr (V > 1) {
-        const int sh0 = o.iz[0] % V;
-        int k = o.iz[0] - sh0;
-#pragma unroll
-        for (int z = 0; z < NV; z++) {
-          iz[z] = k;
-          k = k + V == a.mesh.n[2] ? 0 : k + V;
-        }
-#pragma unroll
-        for (int z = 0; z < NV * V; z++)
-          wz[z] = dz[z] = 0;
-#pragma unroll
-        for (int s = 0; s < V; s++)
-#pragma unroll
-          for (int z = 0; z < P; z++)
-            if (s == sh0) {
-              wz[s + z] = o.wz[z];
-              dz[s + z] = o.dz[z];
-            }
-      } else {
-#pragma unroll
-        for (int z = 0; z < NV; z++) {
-          wz[z] = o.wz[z];
-          dz[z] = o.dz[z];
-          iz[z] = o.iz[z];
-        }
-      }
       // sums of the potential (s0: weights; s1, s2, s3: the derivative along x, y, z)
       // or, with ik, of the potential and the three field meshes
       T s0 = 0, s1 = 0, s2 = 0, s3 = 0;
@@ -216,26 +171,16 @@ __global__ void __launch_bounds__(kSiteThreads, L == 1 ? 6 : 1) k_sites(SiteArgs
           const int row = o.iy[y] * a.mesh.n[2];
           T u0 = 0, u1 = 0, u2 = 0, u3 = 0;
 #pragma unroll
-          for (int z = 0; z < NV; z++) {
-            const int k = row + iz[z];
-            const MeshVec<T, V> u = mesh_load<V>(mp + k);
-            MeshVec<T, V> e1, e2, e3;
+          for (int z = 0; z < NZ; z++) {
+            const int k = row + o.iz[z];
+            const T u = __ldg(mp + k), w = o.wz[z];
+            u0 += w * u;
             if constexpr (kIk) {
-              e1 = mesh_load<V>(ep + k);
-              e2 = mesh_load<V>(ep + a.nr + k);
-              e3 = mesh_load<V>(ep + 2 * a.nr + k);
-            }
-#pragma unroll
-            for (int s = 0; s < V; s++) {
-              const T w = wz[z * V + s];
-              u0 += w * u.v[s];
-              if constexpr (kIk) {
-                u1 += w * e1.v[s];
-                u2 += w * e2.v[s];
-                u3 += w * e3.v[s];
-              } else {
-                u3 += dz[z * V + s] * u.v[s];
-              }
+              u1 += w * __ldg(ep + k);
+              u2 += w * __ldg(ep + a.nr + k);
+              u3 += w * __ldg(ep + 2 * a.nr + k);
+            } else {
+              u3 += o.dz[z] * u;
             }
           }
           t0 += o.wy[y] * u0;
@@ -461,20 +406,21 @@ static int site_grid(int nsite, int L) { return div_up((long) div_up(nsite, 32 /
 
 int site_blocks(const mmnb_handle *h) { return site_grid(h->nsite, kMaxOrder); }
 
-// A lane per mesh plane up to this many sites (a quarter of the chip's threads at
-// one per site); figures above
-constexpr int kSiteLanesMax = 40000;
+// A lane per mesh plane up to this many sites, where a lane per site leaves most of the
+// chip idle; past it the P lanes repeat the weights more often than they hide loads.  The
+// step in us, lanes per plane against per site: order 5 mixed, 6,000 sites 39.4 and 38.2,
+// 9,000 45.1 and 44.3, 16,500 54.3 and 51.0, 33,000 75.4 and 68.5; FP64 47.6 and 49.0,
+// 53.9 and 55.6, 80.1 and 76.3, 119.7 and 110.1; order 7 mixed 43.7 and 48.2, 52.0 and
+// 55.4, 67.3 and 63.6, FP64 56.1 and 54.2, 66.7 and 64.4, 100 and 88.
+constexpr int kSiteLanesMax = 10000;
 
 template <int P, MeshKind KIND>
 static void launch_sites_p(mmnb_handle *h, const SiteArgs &a)
 {
-  constexpr int V = KIND == kMesh32 || KIND == kMesh32Ik ? 4 : 2;
   if (h->nsite <= kSiteLanesMax)
-    k_sites<P, KIND, P, 1><<<site_grid(h->nsite, P), kSiteThreads, 0, h->stream>>>(a);
-  else if (h->mesh[2] % V == 0)
-    k_sites<P, KIND, 1, V><<<site_grid(h->nsite, 1), kSiteThreads, 0, h->stream>>>(a);
+    k_sites<P, KIND, P><<<site_grid(h->nsite, P), kSiteThreads, 0, h->stream>>>(a);
   else
-    k_sites<P, KIND, 1, 1><<<site_grid(h->nsite, 1), kSiteThreads, 0, h->stream>>>(a);
+    k_sites<P, KIND, 1><<<site_grid(h->nsite, 1), kSiteThreads, 0, h->stream>>>(a);
 }
 
 template <MeshKind KIND>
@@ -552,7 +498,7 @@ cudaError_t launch_sites(mmnb_handle *h, const double *d_r, double *d_f, double 
   a.status = h->want_status ? h->d_status : nullptr;
   h->launches += 1;
   if (!p3m) {
-    k_sites<0, kNoMesh, 2, 1><<<site_grid(h->nsite, 2), kSiteThreads, 0, h->stream>>>(a);
+    k_sites<0, kNoMesh, 2><<<site_grid(h->nsite, 2), kSiteThreads, 0, h->stream>>>(a);
     return cudaGetLastError();
   }
   const bool ik = h->cfg.p3m_ik_differentiate != 0;
