@@ -1113,20 +1113,20 @@ int mmnb_compute_device(mmnb_handle *h, const double *d_r, double *d_f, double *
     CK(launch_sort_sites(h, d_r));
   timing_mark(h, "sort_sites");
   h->used_fx = false;
-  h->used_rows64 = false;
+  h->used_rows = false;
   if (h->cfg.include_rspace) {
     if (mixed && h->water && !h->want_fields) {
       CK(launch_rspace_water(h));
       h->used_fx = true;
     } else if (mixed) {
       CK(launch_rspace_mixed(h));
-      h->used_fx = true;
+      h->used_rows = true;
     } else if (water64) {
       CK(launch_rspace_water64(h));
-      h->used_rows64 = true;
+      h->used_rows = true;
     } else {
       CK(launch_rspace_fp64(h));
-      h->used_rows64 = true;
+      h->used_rows = true;
     }
     timing_mark(h, "rspace_pair");
   } else if (mixed) {

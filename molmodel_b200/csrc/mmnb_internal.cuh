@@ -124,8 +124,8 @@ struct mmnb_handle {
   double uni64[4] = {0, 0, 0, 0};    // the same in FP64
   bool want_fields = false;          // this evaluation must produce per-site potential and field
   bool want_virial = false;          // this evaluation's pair kernels also sum the virial's pair term
-  bool used_fx = false;              // the last evaluation ran a mixed pair kernel: fixed-point energies
-  bool used_rows64 = false;          // the last evaluation ran an FP64 pair kernel: energies per row
+  bool used_fx = false;              // the last evaluation ran the mixed water kernel: fixed-point energies
+  bool used_rows = false;            // the last evaluation ran another pair kernel: energies per row
   double totA = 0, totB = 0, lj_correction = 0, neutral_b = 0;
 
   // host topology
@@ -199,17 +199,17 @@ struct mmnb_handle {
 
   // outputs (original order)
   double *d_phi = nullptr, *d_evec = nullptr, *d_ljf = nullptr;
-  double *d_lj_row = nullptr;        // FP64 pair kernels: LJ energy of each row (sorted order)
+  double *d_lj_row = nullptr;        // pair kernels but the mixed water one: LJ energy of each row (sorted order)
   double *d_site_part = nullptr;     // site kernel: per block, its four partial sums
-  // mmnb_virial: the FP64 pair kernels' virial term per row, molecule ranges,
+  // mmnb_virial: the same kernels' virial term per row, molecule ranges,
   // masses and per-molecule sums (allocated on first use)
   double *d_vir_row = nullptr;
   int *d_vir_mol = nullptr;
   double *d_vir_molw = nullptr, *d_vir_mass = nullptr;
   int vir_mol_cap = 0;
-  // [0], [1]: fixed-point Coulomb (rigid water) and LJ pair energies of the mixed pair kernels;
+  // [0], [1]: fixed-point Coulomb and LJ pair energies of the mixed water kernel;
   // [2]: block counter of the site kernel's last-block reduction;
-  // [3]: row counter of the FP64 pair kernels; [4]: the mixed pair kernels'
+  // [3]: row counter of the FP64 pair kernels; [4]: the mixed water kernel's
   // fixed-point virial term
   unsigned long long *d_wsum = nullptr;
   // parameter gradients (allocated on first use): six per-site outputs, dL/dF

@@ -98,7 +98,7 @@ struct MixedArgs {
   const int *nbr, *nbr_count, *sorted;
   const int *gexcl_ptr, *gexcl_idx, *excl_ptr, *excl_idx;
   long long *acc;               // per site, kAccStride
-  unsigned long long *wsum;     // [1]: fixed-point LJ energy, [4]: the virial's pair term
+  double *lj_row, *vir_row;     // per row: LJ energy and (mmnb_virial) the virial's pair term
 };
 
 __device__ __forceinline__ long long to_fx(float v) { return __float2ll_rn(v * 4294967296.0f); }
@@ -281,7 +281,8 @@ __global__ void __launch_bounds__(32, 20) k_pair_mixed(MixedArgs a)
       sum += red[l][c];
     a.acc[(size_t) (si0 + i) * kAccStride + c] = sum;
   }
-  // integer sums: the totals do not depend on the order rows finish in
+  // Per row, added in FP64 and row order by k_sites: a row's energy fits its fixed-point
+  // word (2^31), the total of a box whose molecules overlap (packed, not relaxed) may not.
 #pragma unroll
   for (int c = kNacc; c < kVals; c++) {
     long long sum = red[lane][c];
@@ -289,7 +290,7 @@ __global__ void __launch_bounds__(32, 20) k_pair_mixed(MixedArgs a)
     for (int o = 16; o > 0; o >>= 1)
       sum += __shfl_xor_sync(0xffffffffu, sum, o);
     if (lane == 0)
-      atomicAdd(a.wsum + (c == kNacc ? 1 : 4), (unsigned long long) sum);
+      (c == kNacc ? a.lj_row : a.vir_row)[p] = (double) sum * kFxInv;
   }
 }
 
@@ -1059,7 +1060,8 @@ cudaError_t launch_rspace_mixed(mmnb_handle *h)
   a.excl_ptr = h->d_excl_ptr;
   a.excl_idx = h->d_excl_idx;
   a.acc = h->mx.acc;
-  a.wsum = h->d_wsum;
+  a.lj_row = h->d_lj_row;
+  a.vir_row = h->d_vir_row;
   switch (h->G) {
   case 1: launch_mixed_g<1>(h, a); break;
   case 2: launch_mixed_g<2>(h, a); break;

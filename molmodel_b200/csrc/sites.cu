@@ -54,9 +54,9 @@ struct SiteArgs {
   double *phi, *evec, *ljf, *f;
   // energy reduction
   double *part;                       // per block: q phi, LJ of 1-4 pairs, their virial, LJ of its rows
-  const double *lj_row;               // FP64 pair kernels: per-row LJ energies [0, nrow), or null
+  const double *lj_row;               // per-row LJ energies [0, nrow), or null
   int nrow, any_q;
-  const unsigned long long *wsum;     // mixed pair kernels' fixed-point energies, or null
+  const unsigned long long *wsum;     // mixed water kernel's fixed-point energies, or null
   unsigned long long *counter;        // finished-block counter, left at 0
   int *flags;                         // list flags: counts evaluations finished on cut rows
   double *status;                     // or null: the host call's mapped status block
@@ -486,7 +486,7 @@ cudaError_t launch_sites(mmnb_handle *h, const double *d_r, double *d_f, double 
   a.ljf = h->d_ljf;
   a.f = d_f;
   a.part = h->d_site_part;
-  a.lj_row = h->used_rows64 ? h->d_lj_row : nullptr;
+  a.lj_row = h->used_rows ? h->d_lj_row : nullptr;
   a.nrow = h->ngroup;
   a.any_q = h->any_q ? 1 : 0;
   a.wsum = h->used_fx ? h->d_wsum : nullptr;

@@ -166,10 +166,10 @@ extern "C" int mmnb_virial(mmnb_handle *h, const double *r, int nmol, const int 
     return s;
   if (e)
     *e = en;
-  // X's sums: per row (FP64 pair kernels) or one fixed-point word (mixed pair
-  // kernels), and the 1-4 LJ pairs' sum (intramolecular: they add to X)
+  // X's sums: per row, or one fixed-point word (mixed water kernel), and the 1-4 LJ
+  // pairs' sum (intramolecular: they add to X)
   const double *part = h->d_vir_row;
-  const int npart = h->cfg.include_rspace && h->used_rows64 ? h->ngroup : 0;
+  const int npart = h->cfg.include_rspace && h->used_rows ? h->ngroup : 0;
   const unsigned long long *fixed = h->cfg.include_rspace && h->used_fx ? h->d_wsum + 4 : nullptr;
   double *res = h->d_vir_molw + nmol;
   k_virial_mol<<<div_up(nmol, kVirThreads), kVirThreads, 0, h->stream>>>(nmol, h->d_vir_mol, h->d_vir_mass,
