@@ -354,8 +354,11 @@ extern "C" int mmnb_phi_at_points(mmnb_handle *h, const double *r, int npoint, c
   cudaError_t e = cudaSuccess;
   // wave vectors of kspace_new(kspace_cutoff, .) (src/kspace.c:35-71): the
   // handle's, or with P3M made here once
-  if (c.include_kspace && !h->ew.made && (e = ewald_make(h, h->ew)) != cudaSuccess)
+  if (c.include_kspace && !h->ew.made && (e = ewald_make(h, h->ew)) != cudaSuccess) {
+    if (e == cudaErrorInvalidValue)
+      return esp_fail(h, MMNB_ERR_ARG, "kspace_cutoff is too large");
     return esp_fail(h, MMNB_ERR_CUDA, std::string("potential at points: ") + cudaGetErrorString(e));
+  }
   const int nk = c.include_kspace ? h->ew.nk : 0;
   EspArgs a{};
   a.nsite = h->nsite;

@@ -42,8 +42,11 @@ namespace mmnb {
 
 constexpr int kEwThreads = 256;          // structure factor: wave vectors per block
 constexpr int kEwWarps = 8;              // summing kernel: warps per block of 32 sites
-constexpr int kEwTable = 36 << 10;       // bytes of phase table a block may hold
-constexpr int kEwMaxN = kEwTable / 48 - 1;
+constexpr int kEwTable = 36 << 10;       // bytes of a block's phase tables of more than one site
+// kspace_cutoff from which the wave vectors, 2/3 pi n^3, are more than an int counts; below
+// it one site's table and the structure factor's dipole weights fit the default 48 KB
+constexpr int kEwMaxCut = 1008;
+static_assert(3 * kEwMaxCut * sizeof(double2) + 32 * 3 * sizeof(double) <= (48u << 10), "phase table too large");
 
 struct EwaldArgs {
   int n, nk, nrow, nmax, tile;  // n: sites or points
@@ -277,8 +280,8 @@ cudaError_t ewald_make(mmnb_handle *h, EwaldSum &e)
 {
   ewald_free(e);
   const double kc = h->cfg.kspace_cutoff, n2max = kc * kc + 1e-8;
-  if (kc >= kEwMaxN + 1.0)
-    return cudaErrorInvalidValue;  // about 10^9 wave vectors
+  if (kc >= kEwMaxCut)
+    return cudaErrorInvalidValue;
   const int nmax = std::max(0, (int) floor(kc));
   std::vector<int4> row;
   std::vector<short4> kint;
