@@ -484,8 +484,11 @@ inline int cell_words(int ncell3) { return chunk_at(ncell3) + div_up(ncell3, 1 <
 // what a launch takes passes beside that kernel's work.  On larger boxes the waiting
 // blocks hold room that the mesh work or the pair kernel's first blocks would use.
 // 216 waters' k-sum 83.4 -> 80.3 us, 512 waters' loss gradient 228 -> 215, 6,000 waters
-// with virial 287 -> 275; 32,768 waters mixed 170.2 -> 173.0, FP64 286.4 -> 289.4 us
-// without the limit.
+// with virial 287 -> 275.  The step in us without and with it, mixed: 2,048 waters 41.0 and
+// 39.2, 8,192 66.0 and 64.2, 12,288 78.6 and 76.7, 16,384 107.1 and 107.1, 24,576 111.7 and
+// 112.5; FP64 51.1 and 47.9, 103.6 and 103.1, 127.9 and 127.2, 177.5 and 177.7, 204.9 and
+// 210.2; solution of 4,600 groups 84.7 and 81.3, of 9,000 124.6 and 124.4, of 18,500 207.7
+// and 208.1.
 constexpr int kAfterGroups = 12288;
 
 template <typename... K, typename... A>
