@@ -81,7 +81,8 @@ struct PairArgs {
 // bytes of a warp's queues
 constexpr int p64_warp_bytes(bool screen, bool gexcl, bool vir)
 {
-  return kP64Ring * (16 * 2 + 16 * 4 + 16 * 4 + 8 + (vir ? 16 : 0) + (screen ? 8 : 0) + 4 * 2 + (gexcl ? 4 * 3 : 0));
+  return kP64Ring * (16 * 2 + 16 * 4 + 16 * 4 + 8 + (vir ? 16 : 0) + (screen ? 8 : 0) + 4 * 2 + (gexcl ? 4 * 3 : 0)) +
+         (gexcl ? 8 * kMaxGroup : 0);
 }
 
 // b0 = erfc(eta r)/r and g with b1 = dscale g, b1 = -2 d b0 / d(r^2); seg and f:
@@ -172,6 +173,7 @@ __global__ void __launch_bounds__(32 * kP64Warps, 1) k_pair_fp64(PairArgs a)
   int *const gj = reinterpret_cast<int *>(qrs + (SCREEN ? kP64Ring : 0)), *const gm = gj + kP64Ring;
   // group exclusions: the partner's first site; 1 + site of a queued site that may be excluded
   int *const gs = gm + kP64Ring, *const qx = gs + kP64Ring, *const lx_ = qx + kP64Ring;
+  unsigned long long *const xmask = reinterpret_cast<unsigned long long *>(lx_ + kP64Ring);  // per row site
   // sums of a row: per-lane values over the charged sites' queue, the totals over the LJ sites'
   double *const red = reinterpret_cast<double *>(q0);
   double *const tot = reinterpret_cast<double *>(l0);
@@ -198,6 +200,14 @@ __global__ void __launch_bounds__(32 * kP64Warps, 1) k_pair_fp64(PairArgs a)
     const long long info = __double_as_longlong(ai.w);
     const int si0 = (int) (info >> 32), ns = (int) info & 0xff, qm = ((int) info >> 8) & 0xff,
               lm = ((int) info >> 16) & 0xff;
+    // sites excluded in other groups: whether any; where the row's lists are (first: what
+    // the row's set-up waits for)
+    const bool row_gx = GEXCL && ((int) info >> 24) & 1;
+    int xb = 0, xe = 0;
+    if (row_gx && lane < ns) {
+      xb = a.excl_ptr[si0 + lane];
+      xe = a.excl_ptr[si0 + lane + 1];
+    }
     const int cnt = a.nbr_count[p];
     const int *row = a.nbr + (size_t) p * a.rowcap;
     const int step = 32 * split;
@@ -216,12 +226,40 @@ __global__ void __launch_bounds__(32 * kP64Warps, 1) k_pair_fp64(PairArgs a)
     const double4 vq = a.sr[(size_t) p * a.G + kq], vl = a.sr[(size_t) p * a.G + kl];
     const double4 pl = a.sp[(size_t) p * a.G + kl];
     const double rsi = SCREEN ? a.sp[(size_t) p * a.G + kq].z : 0.0;
-    int gi = 0;
-    bool row_gx = false;
-    if (GEXCL) {
-      gi = a.sorted[p];
-      row_gx = a.gexcl_ptr[gi + 1] > a.gexcl_ptr[gi];
+    // The first and the last site that any site of the row excludes.  Up to 64 sites apart,
+    // each row site's as a mask from the first on; a row of one site then drops what it
+    // excludes before the queues.  (A search per partner and per site pair, chains of
+    // dependent loads that the other lanes wait for, in chains of 64,000 single sites that
+    // exclude three to each side: the pair kernel 1247 us, 820 so.)
+    int xlo = 1 << 30, xhi = -1;
+    unsigned long long xone = 0;
+    if (row_gx) {
+      if (xb < xe) {
+        xlo = a.excl_idx[xb];
+        xhi = a.excl_idx[xe - 1];
+      }
+      xlo = __reduce_min_sync(0xffffffffu, xlo);
+      xhi = __reduce_max_sync(0xffffffffu, xhi);
     }
+    const bool masks = xhi - xlo < 64, single = masks && ns == 1;
+    if (row_gx && single) {
+      const int b = __shfl_sync(0xffffffffu, xb, 0), e = __shfl_sync(0xffffffffu, xe, 0);
+      for (int n = b + lane; n < e; n += 32)
+        xone |= 1ull << (a.excl_idx[n] - xlo);
+      xone = (unsigned long long) __reduce_or_sync(0xffffffffu, (unsigned) (xone >> 32)) << 32 |
+             __reduce_or_sync(0xffffffffu, (unsigned) xone);
+    } else if (row_gx && masks && lane < ns) {
+      unsigned long long m = 0;
+      for (int n = xb; n < xe; n++)
+        m |= 1ull << (a.excl_idx[n] - xlo);
+      xmask[lane] = m;
+    }
+    const bool late = row_gx && !single;  // site pairs are looked at in the queues
+    // whether site k of the row excludes site j
+    auto excluded = [&](int k, int j) {
+      return masks ? (unsigned) (j - xlo) < 64u && (xmask[k] >> (j - xlo)) & 1
+                   : csr_has(a.excl_ptr, a.excl_idx, si0 + k, j);
+    };
     double ph = 0, ex = 0, ey = 0, ez = 0, sx = 0, sy = 0, sz = 0;  // charges; s: switch force / q_i
     double lx = 0, ly = 0, lz = 0, tx = 0, ty = 0, tz = 0, elj = 0, vir = 0;
     int gh = 0, gn = 0, qh = 0, qn = 0, lh = 0, ln = 0;
@@ -240,10 +278,12 @@ __global__ void __launch_bounds__(32 * kP64Warps, 1) k_pair_fp64(PairArgs a)
           ga[k] = make_double2(x, y);
           gb[k] = make_double2(z, r2a);
           gj[k] = jc;
-          int m = (int) __double_as_longlong(ac.w);
-          if (GEXCL && row_gx) {
-            gs[k] = (int) (__double_as_longlong(ac.w) >> 32);
-            if (csr_has(a.gexcl_ptr, a.gexcl_idx, gi, a.sorted[jc]))
+          int m = (int) __double_as_longlong(ac.w) & 0xffffff;
+          if (row_gx) {
+            const int s0 = (int) (__double_as_longlong(ac.w) >> 32);
+            gs[k] = s0;
+            if (s0 <= xhi && s0 + (m & 0xff) > xlo &&
+                (masks || csr_has(a.gexcl_ptr, a.gexcl_idx, a.sorted[p], a.sorted[jc])))
               m |= 1 << 24;
           }
           gm[k] = m;
@@ -270,8 +310,10 @@ __global__ void __launch_bounds__(32 * kP64Warps, 1) k_pair_fp64(PairArgs a)
           s = a.sr[slot];
           if (SCREEN || (em & 2))
             sp = a.sp[slot];
-          if (GEXCL && (m >> 24) & 1)
-            em |= 4;
+          if (GEXCL && (m >> 24) & 1) {
+            const unsigned d = gs[k] + ek - xlo;
+            em = !single ? em | 4 : d < 64 && (xone >> d) & 1 ? 0 : em;
+          }
         }
       }
     };
@@ -294,7 +336,7 @@ __global__ void __launch_bounds__(32 * kP64Warps, 1) k_pair_fp64(PairArgs a)
             qg[e] = ds * zr.y;
           if (SCREEN)
             qrs[e] = sp.z;
-          if (GEXCL && row_gx)
+          if (late)
             qx[e] = em & 4 ? gs[k] + ek + 1 : 0;
         }
         if (em & 2) {
@@ -306,7 +348,7 @@ __global__ void __launch_bounds__(32 * kP64Warps, 1) k_pair_fp64(PairArgs a)
           l4[e] = ds * zr.x;
           if (VIR)
             lg[e] = ds * zr.y;
-          if (GEXCL && row_gx)
+          if (late)
             lx_[e] = em & 4 ? gs[k] + ek + 1 : 0;
         }
       }
@@ -320,7 +362,7 @@ __global__ void __launch_bounds__(32 * kP64Warps, 1) k_pair_fp64(PairArgs a)
       if (aq && sq < n) {
         const int e = (qh + sq) & kMask;
         const double2 e0 = q0[e], e1 = q1[e], e2 = q2[e], e3 = q3[e];
-        const bool out = GEXCL && row_gx && qx[e] && csr_has(a.excl_ptr, a.excl_idx, si0 + kq, qx[e] - 1);
+        const bool out = late && qx[e] && excluded(kq, qx[e] - 1);
         if (!out) {
           const double dx = vq.x - e0.x, dy = vq.y - e0.y, dz = vq.z - e1.x;
           const double r2 = dx * dx + dy * dy + dz * dz;
@@ -364,7 +406,7 @@ __global__ void __launch_bounds__(32 * kP64Warps, 1) k_pair_fp64(PairArgs a)
         const int e = (lh + sl) & kMask;
         const double2 e0 = l0[e], e1 = l1[e], e2 = l2[e], e3 = l3[e];
         const double gz = l4[e];
-        const bool out = GEXCL && row_gx && lx_[e] && csr_has(a.excl_ptr, a.excl_idx, si0 + kl, lx_[e] - 1);
+        const bool out = late && lx_[e] && excluded(kl, lx_[e] - 1);
         if (!out) {
           const double dx = vl.x - e0.x, dy = vl.y - e0.y, dz = vl.z - e1.x;
           const double ir2 = 1.0 / (dx * dx + dy * dy + dz * dz);
@@ -494,11 +536,13 @@ __global__ void __launch_bounds__(32 * kP64Warps, 1) k_pair_fp64(PairArgs a)
 // Sorted FP64 site data for the pair kernel: slots of (offset from the anchor,
 // charge) and (sigma, sqrt(epsilon), r_screen, -), and per group the anchor with
 // its first site (high word) and number of sites, charged sites and LJ sites (a
-// byte each of the low word: bit k for site k).  Clears the row counter.
+// byte each of the low word: bit k for site k), and bit 24 for exclusions across groups
+// (gexcl_ptr, or null without any).  Clears the row counter.
 __device__ __forceinline__ void sort_sites(const double *__restrict__ r, const double *__restrict__ q,
                              const double *__restrict__ sig, const double *__restrict__ eps,
                              const double *__restrict__ rscreen, const int *__restrict__ mask,
-                             const int *__restrict__ sorted, const int *__restrict__ group, int ngroup, int G,
+                             const int *__restrict__ sorted, const int *__restrict__ group,
+                             const int *__restrict__ gexcl_ptr, int ngroup, int G,
                              double4 *__restrict__ sr, double4 *__restrict__ sp, double4 *__restrict__ anchor,
                              unsigned long long *__restrict__ counter, int *__restrict__ flags)
 {
@@ -513,6 +557,8 @@ __device__ __forceinline__ void sort_sites(const double *__restrict__ r, const d
   const double ax = r[3 * s0], ay = r[3 * s0 + 1], az = r[3 * s0 + 2];
   if (k == 0) {
     unsigned m = n;
+    if (gexcl_ptr && gexcl_ptr[g + 1] > gexcl_ptr[g])
+      m |= 1u << 24;
     for (int j = 0; j < n; j++) {
       const int b = mask[s0 + j];
       m |= (b & MMNB_SITE_HAS_Q ? 1u << (8 + j) : 0u) | (b & MMNB_SITE_HAS_LJ ? 1u << (16 + j) : 0u);
@@ -532,12 +578,12 @@ __device__ __forceinline__ void sort_sites(const double *__restrict__ r, const d
 __global__ void __launch_bounds__(32 * kRowWarps)
 k_sort_sites(const double *__restrict__ r, const double *__restrict__ q, const double *__restrict__ sig,
              const double *__restrict__ eps, const double *__restrict__ rscreen, const int *__restrict__ mask,
-             const int *__restrict__ sorted, const int *__restrict__ group, int ngroup, int G,
-             double4 *__restrict__ sr, double4 *__restrict__ sp, double4 *__restrict__ anchor,
+             const int *__restrict__ sorted, const int *__restrict__ group, const int *__restrict__ gexcl_ptr,
+             int ngroup, int G, double4 *__restrict__ sr, double4 *__restrict__ sp, double4 *__restrict__ anchor,
              unsigned long long *__restrict__ counter, int *__restrict__ flags, RebuildArgs rows)
 {
   after_previous();
-  sort_sites(r, q, sig, eps, rscreen, mask, sorted, group, ngroup, G, sr, sp, anchor, counter, flags);
+  sort_sites(r, q, sig, eps, rscreen, mask, sorted, group, gexcl_ptr, ngroup, G, sr, sp, anchor, counter, flags);
   build_rows(rows);
 }
 
@@ -545,8 +591,8 @@ cudaError_t launch_sort_sites(mmnb_handle *h, const double *d_r)
 {
   const int n = h->ngroup * h->G;
   launch_after(h, k_sort_sites, sort_blocks(h, n), 32 * kRowWarps, 0, d_r, h->d_q, h->d_sig, h->d_eps,
-               h->d_rscreen, h->d_mask, h->d_sorted, h->d_group, h->ngroup, h->G, h->d_sr, h->d_sp, h->d_sanchor,
-               h->d_wsum + 3, h->d_flags, rebuild_args(h));
+               h->d_rscreen, h->d_mask, h->d_sorted, h->d_group, h->any_gexcl ? h->d_gexcl_ptr : nullptr,
+               h->ngroup, h->G, h->d_sr, h->d_sp, h->d_sanchor, h->d_wsum + 3, h->d_flags, rebuild_args(h));
   h->launches += 1;
   return cudaGetLastError();
 }
