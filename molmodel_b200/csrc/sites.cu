@@ -105,6 +105,36 @@ __device__ __forceinline__ void excluded_b(const SiteArgs &a, double r2, double 
   }
 }
 
+// a mesh row's points of one lane, 16 bytes a load when whole rows allow it
+template <typename T, int V>
+struct MeshVec {
+  T v[V];
+};
+template <int V>
+__device__ __forceinline__ MeshVec<float, V> mesh_load(const float *p)
+{
+  MeshVec<float, V> o;
+  if constexpr (V == 4) {
+    const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
+    o.v[0] = t.x, o.v[1] = t.y, o.v[2] = t.z, o.v[3] = t.w;
+  } else {
+    o.v[0] = __ldg(p);
+  }
+  return o;
+}
+template <int V>
+__device__ __forceinline__ MeshVec<double, V> mesh_load(const double *p)
+{
+  MeshVec<double, V> o;
+  if constexpr (V == 2) {
+    const double2 t = __ldg(reinterpret_cast<const double2 *>(p));
+    o.v[0] = t.x, o.v[1] = t.y;
+  } else {
+    o.v[0] = __ldg(p);
+  }
+  return o;
+}
+
 // Blocks an SM the register budget is cut for, a lane per site.  The sites' loads want
 // many warps, a spilled order takes more from them than they give, and the best cut
 // moves with the order's arrays.  32,768 waters, the step in us at 6 / 4 / 3 / 2 blocks:
@@ -118,15 +148,33 @@ __device__ __forceinline__ void excluded_b(const SiteArgs &a, double r2, double 
 // (orders 5 and 7 of 66,000 sites with ik, mixed: one wave at 4 blocks, 149 us; 154 at
 // 6, 163 at 3.)  One cap of 6 for all, which order 5's whole-word rows were measured
 // with, spilled up to 6 KB a thread: order 7 388 us FP64 and 233 mixed on rows of 81.
-constexpr int site_blocks_per_sm(int P, MeshKind kind)
+constexpr int site_blocks_per_sm(int P, MeshKind kind, int V)
 {
   const bool k32 = kind == kMesh32 || kind == kMesh32Ik, ik = kind == kMesh64Ik || kind == kMesh32Ik;
+  if (V > 1)
+    return k32 || P <= 5 ? 6 : 3;
   return P <= 3 || (k32 && P == 4) ? 6 : P == 4 || (k32 && P == 5) ? 4 : !k32 && (P == 7 || ik) ? 2 : 3;
 }
 
-// P: assignment order, or 0 without a mesh; L: lanes per site (P or one with a mesh)
-template <int P, MeshKind KIND, int L>
-__global__ void __launch_bounds__(kSiteThreads, L == 1 ? site_blocks_per_sm(P, KIND) : 1) k_sites(SiteArgs a)
+// Mesh points a load of a lane per site past kSiteWordsMin sites.  16 bytes' take fewer
+// requests of a row but 8 points for an order of 5: little in a box whose molecules are in
+// order, more once they have diffused and a warp's sites share no lines.  32,768 waters in
+// order / shuffled, us a step, point by point and by 16 bytes: order 5 mixed 147 / 161 and
+// 147 / 150; with ik, mixed 4 180 / 226 and 189 / 205, 5 207 / 272 and 205 / 231; FP64 4
+// 348 / 375 and 347 / 366, 5 368 / 417 and 369 / 404, 7 470 / 612 and 472 / 565.  The others
+// point by point: order 7 mixed 192 / 217 and 198 / 211, with ik 269 / 395 and 294 / 367,
+// 3 with ik 160 / 183 and 168 / 179, FP64 6 288 / 306 and 290 / 300.
+constexpr int site_words(int P, MeshKind kind)
+{
+  if (kind == kMesh64Ik)
+    return P >= 4 ? 2 : 1;
+  return (kind == kMesh32 && P == 5) || (kind == kMesh32Ik && (P == 4 || P == 5)) ? 4 : 1;
+}
+
+// P: assignment order, or 0 without a mesh; L: lanes per site (P or one with a mesh);
+// V: mesh points per load (one lane per site and rows of whole 16-byte words; else 1)
+template <int P, MeshKind KIND, int L, int V>
+__global__ void __launch_bounds__(kSiteThreads, L == 1 ? site_blocks_per_sm(P, KIND, V) : 1) k_sites(SiteArgs a)
 {
   constexpr int S = 32 / L;
   constexpr bool k32 = KIND == kMesh32 || KIND == kMesh32Ik, kIk = KIND == kMesh64Ik || KIND == kMesh32Ik;
@@ -154,10 +202,42 @@ __global__ void __launch_bounds__(kSiteThreads, L == 1 ? site_blocks_per_sm(P, K
     if constexpr (KIND != kNoMesh) {
       typedef typename std::conditional<k32, float, double>::type T;
       constexpr int NZ = L == 1 ? P : 1;  // points along z of this lane
+      constexpr int NV = V == 1 ? NZ : (V - 1 + P + V - 1) / V;  // loads a row
       MeshRows<P, NZ, T> o;
       mesh_rows<P, NZ, T>(a.mesh, a.r + 3 * (size_t) i, c, o);
       const T *const mesh = k32 ? (const T *) a.mesh32 : (const T *) a.mesh64;
       const T *const eg = k32 ? (const T *) a.egrid32 : (const T *) a.egrid64;
+      // the row's words and the weights of their points: with whole words the P points
+      // start at point `sh0` of the first, the others weigh nothing
+      T wz[NV * V], dz[NV * V];
+      int iz[NV];
+      if constexpr (V > 1) {
+        const int sh0 = o.iz[0] % V;
+        int k = o.iz[0] - sh0;
+#pragma unroll
+        for (int z = 0; z < NV; z++) {
+          iz[z] = k;
+          k = k + V == a.mesh.n[2] ? 0 : k + V;
+        }
+#pragma unroll
+        for (int z = 0; z < NV * V; z++)
+          wz[z] = dz[z] = 0;
+#pragma unroll
+        for (int s = 0; s < V; s++)
+#pragma unroll
+          for (int z = 0; z < P; z++)
+            if (s == sh0) {
+              wz[s + z] = o.wz[z];
+              dz[s + z] = o.dz[z];
+            }
+      } else {
+#pragma unroll
+        for (int z = 0; z < NV; z++) {
+          wz[z] = o.wz[z];
+          dz[z] = o.dz[z];
+          iz[z] = o.iz[z];
+        }
+      }
       // sums of the potential (s0: weights; s1, s2, s3: the derivative along x, y, z)
       // or, with ik, of the potential and the three field meshes
       T s0 = 0, s1 = 0, s2 = 0, s3 = 0;
@@ -171,16 +251,26 @@ __global__ void __launch_bounds__(kSiteThreads, L == 1 ? site_blocks_per_sm(P, K
           const int row = o.iy[y] * a.mesh.n[2];
           T u0 = 0, u1 = 0, u2 = 0, u3 = 0;
 #pragma unroll
-          for (int z = 0; z < NZ; z++) {
-            const int k = row + o.iz[z];
-            const T u = __ldg(mp + k), w = o.wz[z];
-            u0 += w * u;
+          for (int z = 0; z < NV; z++) {
+            const int k = row + iz[z];
+            const MeshVec<T, V> u = mesh_load<V>(mp + k);
+            MeshVec<T, V> e1, e2, e3;
             if constexpr (kIk) {
-              u1 += w * __ldg(ep + k);
-              u2 += w * __ldg(ep + a.nr + k);
-              u3 += w * __ldg(ep + 2 * a.nr + k);
-            } else {
-              u3 += o.dz[z] * u;
+              e1 = mesh_load<V>(ep + k);
+              e2 = mesh_load<V>(ep + a.nr + k);
+              e3 = mesh_load<V>(ep + 2 * a.nr + k);
+            }
+#pragma unroll
+            for (int s = 0; s < V; s++) {
+              const T w = wz[z * V + s];
+              u0 += w * u.v[s];
+              if constexpr (kIk) {
+                u1 += w * e1.v[s];
+                u2 += w * e2.v[s];
+                u3 += w * e3.v[s];
+              } else {
+                u3 += dz[z * V + s] * u.v[s];
+              }
             }
           }
           t0 += o.wy[y] * u0;
@@ -413,14 +503,20 @@ int site_blocks(const mmnb_handle *h) { return site_grid(h->nsite, kMaxOrder); }
 // 53.9 and 55.6, 80.1 and 76.3, 119.7 and 110.1; order 7 mixed 43.7 and 48.2, 52.0 and
 // 55.4, 67.3 and 63.6, FP64 56.1 and 54.2, 66.7 and 64.4, 100 and 88.
 constexpr int kSiteLanesMax = 10000;
+// (site_words' loads, at 6 blocks an SM, want the chip filled: order 5 mixed, shuffled, point
+// by point against them: 18,000 sites 58.0 and 60.8, 36,000 74.7 and 75.1, 98,304 161 and 150)
+constexpr int kSiteWordsMin = 40000;
 
 template <int P, MeshKind KIND>
 static void launch_sites_p(mmnb_handle *h, const SiteArgs &a)
 {
+  constexpr int V = site_words(P, KIND);
   if (h->nsite <= kSiteLanesMax)
-    k_sites<P, KIND, P><<<site_grid(h->nsite, P), kSiteThreads, 0, h->stream>>>(a);
+    k_sites<P, KIND, P, 1><<<site_grid(h->nsite, P), kSiteThreads, 0, h->stream>>>(a);
+  else if (h->nsite > kSiteWordsMin && h->mesh[2] % V == 0)
+    k_sites<P, KIND, 1, V><<<site_grid(h->nsite, 1), kSiteThreads, 0, h->stream>>>(a);
   else
-    k_sites<P, KIND, 1><<<site_grid(h->nsite, 1), kSiteThreads, 0, h->stream>>>(a);
+    k_sites<P, KIND, 1, 1><<<site_grid(h->nsite, 1), kSiteThreads, 0, h->stream>>>(a);
 }
 
 template <MeshKind KIND>
@@ -498,7 +594,7 @@ cudaError_t launch_sites(mmnb_handle *h, const double *d_r, double *d_f, double 
   a.status = h->want_status ? h->d_status : nullptr;
   h->launches += 1;
   if (!p3m) {
-    k_sites<0, kNoMesh, 2><<<site_grid(h->nsite, 2), kSiteThreads, 0, h->stream>>>(a);
+    k_sites<0, kNoMesh, 2, 1><<<site_grid(h->nsite, 2), kSiteThreads, 0, h->stream>>>(a);
     return cudaGetLastError();
   }
   const bool ik = h->cfg.p3m_ik_differentiate != 0;
