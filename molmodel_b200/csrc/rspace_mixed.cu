@@ -107,9 +107,11 @@ __device__ __forceinline__ long long to_fx(float v) { return __float2ll_rn(v * 4
 // leaves no division, shuffle or inner loop and registers for all 32 blocks an SM takes: the
 // step of 97,336 single sites (305 partners within rc) 718 us with a lane per partner
 // group's padded sites, 757 in this layout with the counts as data, 570 so (633 at 20
-// blocks, 591 at 24); 27,000 of them 195, 212 and 173.
+// blocks, 591 at 24); 27,000 of them 195, 212 and 173.  With exclusions across groups cut
+// for 24: 1,700 sites in molecules of 40 65 us (71 at 32 blocks, 66 before), 27,000 340
+// (323 and 368).
 template <int G, bool SCREEN, bool GEXCL, bool VIR>
-__global__ void __launch_bounds__(32, G == 1 ? 32 : 20) k_pair_mixed(MixedArgs a)
+__global__ void __launch_bounds__(32, G > 1 ? 20 : GEXCL ? 24 : 32) k_pair_mixed(MixedArgs a)
 {
   after_previous();
   constexpr int kMask = kMxQueue - 1, kVals = kNacc + (VIR ? 2 : 1);
