@@ -918,15 +918,12 @@ int mmnb_set_params(mmnb_handle *h, const int *site_mask, const double *q, const
   h->buf_gen++;  // the kernels an evaluation launches may change
   const int n = h->nsite;
   h->any_q = h->any_lj = h->has_rscreen = false;
-  h->lj_on_anchors_only = true;
   double qsum = 0;
   for (int i = 0; i < n; i++) {
     if (site_mask[i] & MMNB_SITE_HAS_Q)
       h->any_q = true;
     if (site_mask[i] & MMNB_SITE_HAS_LJ) {
       h->any_lj = true;
-      if (h->group[2 * h->group_of_site[i]] != i)
-        h->lj_on_anchors_only = false;
       if (!(sig[i] > 0) || eps[i] < 0)
         return fail(h, MMNB_ERR_ARG, "LJ sites need sigma > 0 and epsilon >= 0");
     }

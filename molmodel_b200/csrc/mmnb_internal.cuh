@@ -115,7 +115,6 @@ struct mmnb_handle {
   double volume = 0, min_diameter = 0;
   bool params_set = false, any_q = false, any_lj = false, has_rscreen = false;
   bool any_gexcl = false, use_14 = false;
-  bool lj_on_anchors_only = false;   // every LJ site is its group's first site (rigid water)
   bool water = false;                // every group is [O(q, LJ), H(q), H(q)] with no screening or group exclusions
   // ... and every O has the same charge, sigma and epsilon and every H the
   // same charge (the rigid-water kernel then copies only the H offsets)

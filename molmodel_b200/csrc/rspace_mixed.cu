@@ -475,23 +475,6 @@ __device__ __forceinline__ void water_site2(f2 dx, f2 dy, f2 dz, f2 qb, f2 qbs, 
   ez = fma2(f, dz, ez);
 }
 
-// Minimum-image anchor displacement with contracted FP64 arithmetic (fewer
-// instructions than the reference-rounded form the FP64 kernels use).  The
-// decision it feeds only matters at r = rc, where the switch and its
-// derivative are zero, so the pair set may differ from the FP64 form's only
-// by pairs that contribute nothing.
-__device__ __forceinline__ double anchor_disp_fast(const Box &b, double4 ri, double4 rj, double &x, double &y,
-                                                   double &z)
-{
-  x = ri.x - rj.x;
-  y = ri.y - rj.y;
-  z = ri.z - rj.z;
-  x = fma(-b.L[0], rint(x * b.invL[0]), x);
-  y = fma(-b.L[1], rint(y * b.invL[1]), y);
-  z = fma(-b.L[2], rint(z * b.invL[2]), z);
-  return fma(x, x, fma(y, y, z * z));
-}
-
 __device__ __forceinline__ void cp_async16(void *dst, const void *src)
 {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"((unsigned) __cvta_generic_to_shared(dst)),
