@@ -760,6 +760,9 @@ static int batch_capture(mmnb_md_batch *b)
   if (e != cudaSuccess)
     return batch_fail(b, MMNB_ERR_CUDA, cudaGetErrorString(e));
   int s = MMNB_OK;
+  long groups = 0;
+  for (const mmnb_md *md : b->md)
+    groups += md->h->ngroup;
   e = cudaEventRecord(b->fork, b->master);
   for (size_t i = 0; i < b->md.size() && e == cudaSuccess && !s; i++) {
     mmnb_md *md = b->md[i];
@@ -768,7 +771,9 @@ static int batch_capture(mmnb_md_batch *b)
     if (e != cudaSuccess)
       break;
     h->capturing = true;
+    h->crowded = groups > kAfterGroups;
     s = md_record(md, md->d_log);
+    h->crowded = false;
     h->capturing = false;
     if (s)
       break;

@@ -103,6 +103,41 @@ __device__ __forceinline__ void mesh_rows(const MeshArgs &m, const double *__res
   }
 }
 
+// The same for a particle's P lanes from lane `first` of the warp on, lane c taking the
+// point z = base + c: three of them work out an axis each and hand it to the others
+// (every lane of the warp calls).
+template <int P, typename T>
+__device__ __forceinline__ void mesh_rows_lanes(const MeshArgs &m, const double *__restrict__ r, int first, int c,
+                                                MeshRows<P, 1, T> &o)
+{
+  const int d = c < 2 ? c : 2;
+  T W[P], D[P];
+  double w;
+  const int b = bspline_base<P>(m.A[d] * r[0] + m.A[3 + d] * r[1] + m.A[6 + d] * r[2], w);
+  bspline_eval<P, T>((T) w, W, D);
+  const int j = wrap_idx(b, m.n[d]);
+  const unsigned all = 0xffffffffu;
+  int jx = __shfl_sync(all, j, first), jy = __shfl_sync(all, j, first + 1), jz = __shfl_sync(all, j, first + 2);
+#pragma unroll
+  for (int p = 0; p < P; p++) {
+    o.ix[p] = jx;
+    o.iy[p] = jy;
+    jx = jx + 1 == m.n[0] ? 0 : jx + 1;
+    jy = jy + 1 == m.n[1] ? 0 : jy + 1;
+    o.wx[p] = __shfl_sync(all, W[p], first);
+    o.dx[p] = __shfl_sync(all, D[p], first);
+    o.wy[p] = __shfl_sync(all, W[p], first + 1);
+    o.dy[p] = __shfl_sync(all, D[p], first + 1);
+    const T wz = __shfl_sync(all, W[p], first + 2), dz = __shfl_sync(all, D[p], first + 2);
+    if (p == c) {
+      o.wz[0] = wz;
+      o.dz[0] = dz;
+      o.iz[0] = jz;
+    }
+    jz = jz + 1 == m.n[2] ? 0 : jz + 1;
+  }
+}
+
 // sum of v over the L lanes [first, first + L) of a particle, into its first lane
 // (c: the lane's place among them; every lane of the warp calls)
 template <int L, typename T>

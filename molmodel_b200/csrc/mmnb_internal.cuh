@@ -303,6 +303,7 @@ struct mmnb_handle {
   bool want_status = false;    // set while the host call records its evaluation: no
                                // other evaluation writes the block
   bool capturing = false;
+  bool crowded = false;  // set while a batch of many replicas records this one's step
 };
 
 namespace mmnb {
@@ -487,7 +488,8 @@ inline int cell_words(int ncell3) { return chunk_at(ncell3) + div_up(ncell3, 1 <
 // 39.2, 8,192 66.0 and 64.2, 12,288 78.6 and 76.7, 16,384 107.1 and 107.1, 24,576 111.7 and
 // 112.5; FP64 51.1 and 47.9, 103.6 and 103.1, 127.9 and 127.2, 177.5 and 177.7, 204.9 and
 // 210.2; solution of 4,600 groups 84.7 and 81.3, of 9,000 124.6 and 124.4, of 18,500 207.7
-// and 208.1.
+// and 208.1.  A batch of replicas that are more than this together does without it (64 of
+// them 766 -> 759 ms per 1,000 steps).
 constexpr int kAfterGroups = 12288;
 
 template <typename... K, typename... A>
@@ -503,7 +505,7 @@ inline cudaError_t launch_after(const mmnb_handle *h, void (*kernel)(K...), dim3
   c.dynamicSmemBytes = smem;
   c.stream = h->stream;
   c.attrs = &at;
-  c.numAttrs = h->ngroup <= kAfterGroups ? 1 : 0;
+  c.numAttrs = h->ngroup <= kAfterGroups && !h->crowded ? 1 : 0;
   return cudaLaunchKernelEx(&c, kernel, K(args)...);
 }
 #endif

@@ -5,7 +5,8 @@
 // (src/eleclj.cpp:794-805, 961-976).
 //
 //   * mesh: P lanes per site along z, lane c taking the points z = base + c of the
-//     site's P^2 rows, so a site's lanes read consecutive mesh words; the P rows of
+//     site's P^2 rows, so a site's lanes read consecutive mesh words (three of them work
+//     out the weights of an axis each for all); the P rows of
 //     one x-plane are summed with the y weights first (2 multiply-adds a point
 //     where the three-weight products of a thread per site took 8).  FP64, or FP32
 //     converted to fixed point per site (mixed form).  Without a mesh, two lanes per
@@ -189,6 +190,12 @@ __global__ void __launch_bounds__(kSiteThreads, L == 1 ? site_blocks_per_sm(P, K
   float v32[4] = {0.f, 0.f, 0.f, 0.f};
   int mi = 0, x0 = 0, x1 = 0, jx = 0;
   double qi = 0;
+  typedef typename std::conditional<k32, float, double>::type T;
+  constexpr int NZ = L == 1 ? P : 1;  // points along z of this lane
+  constexpr bool kShared = KIND != kNoMesh && L >= 3;
+  MeshRows<P ? P : 1, P ? NZ : 1, T> o;
+  if constexpr (kShared)
+    mesh_rows_lanes<P, T>(a.mesh, a.r + 3 * (size_t) (live ? i : 0), lane - c, c, o);
   if (live) {
     // first what the later parts' loads depend on
     mi = a.mask[i];
@@ -200,11 +207,9 @@ __global__ void __launch_bounds__(kSiteThreads, L == 1 ? site_blocks_per_sm(P, K
         jx = a.excl_idx[x0];
     }
     if constexpr (KIND != kNoMesh) {
-      typedef typename std::conditional<k32, float, double>::type T;
-      constexpr int NZ = L == 1 ? P : 1;  // points along z of this lane
       constexpr int NV = V == 1 ? NZ : (V - 1 + P + V - 1) / V;  // loads a row
-      MeshRows<P, NZ, T> o;
-      mesh_rows<P, NZ, T>(a.mesh, a.r + 3 * (size_t) i, c, o);
+      if constexpr (!kShared)
+        mesh_rows<P, NZ, T>(a.mesh, a.r + 3 * (size_t) i, c, o);
       const T *const mesh = k32 ? (const T *) a.mesh32 : (const T *) a.mesh64;
       const T *const eg = k32 ? (const T *) a.egrid32 : (const T *) a.egrid64;
       // the row's words and the weights of their points: with whole words the P points
@@ -497,12 +502,15 @@ static int site_grid(int nsite, int L) { return div_up((long) div_up(nsite, 32 /
 int site_blocks(const mmnb_handle *h) { return site_grid(h->nsite, kMaxOrder); }
 
 // A lane per mesh plane up to this many sites, where a lane per site leaves most of the
-// chip idle; past it the P lanes repeat the weights more often than they hide loads.  The
-// step in us, lanes per plane against per site: order 5 mixed, 6,000 sites 39.4 and 38.2,
-// 9,000 45.1 and 44.3, 16,500 54.3 and 51.0, 33,000 75.4 and 68.5; FP64 47.6 and 49.0,
-// 53.9 and 55.6, 80.1 and 76.3, 119.7 and 110.1; order 7 mixed 43.7 and 48.2, 52.0 and
-// 55.4, 67.3 and 63.6, FP64 56.1 and 54.2, 66.7 and 64.4, 100 and 88.
-constexpr int kSiteLanesMax = 10000;
+// chip idle.  The step in us, lanes per plane against per site: order 5 mixed, 650 sites
+// 28.0 and 29.9, 3,000 32.8 and 34.9, 8,700 42.1 and 43.5; with ik 1,500 32.4 and 37.5;
+// order 7 3,000 36.9 and 42.8; FP64 order 5 3,000 34.9 and 36.9, 8,700 53.8 and 55.4, order 7
+// 38.7 and 43.1, 62.5 and 64.4.  Past it (the weights repeated in each lane) order 5 mixed,
+// 16,500 sites 54.3 and 51.0, 33,000 75.4 and 68.5; FP64 80.1 and 76.3, 119.7 and 110.1.
+// Mixed orders up to 5 without ik, where the lanes gain least, take a lane per site from
+// 2,500 sites on: replicas that fill the chip together pay for the lanes' work (64 of 258
+// to 3,933 waters, 1,000 steps: 760 ms with 10,000 here, 731 with 2,500).
+constexpr int site_lanes_max(int P, MeshKind kind) { return kind == kMesh32 && P <= 5 ? 2500 : 10000; }
 // (site_words' loads, at 6 blocks an SM, want the chip filled: order 5 mixed, shuffled, point
 // by point against them: 18,000 sites 58.0 and 60.8, 36,000 74.7 and 75.1, 98,304 161 and 150)
 constexpr int kSiteWordsMin = 40000;
@@ -511,7 +519,7 @@ template <int P, MeshKind KIND>
 static void launch_sites_p(mmnb_handle *h, const SiteArgs &a)
 {
   constexpr int V = site_words(P, KIND);
-  if (h->nsite <= kSiteLanesMax)
+  if (h->nsite <= site_lanes_max(P, KIND))
     k_sites<P, KIND, P, 1><<<site_grid(h->nsite, P), kSiteThreads, 0, h->stream>>>(a);
   else if (h->nsite > kSiteWordsMin && h->mesh[2] % V == 0)
     k_sites<P, KIND, 1, V><<<site_grid(h->nsite, 1), kSiteThreads, 0, h->stream>>>(a);
