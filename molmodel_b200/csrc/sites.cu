@@ -501,16 +501,20 @@ static int site_grid(int nsite, int L) { return div_up((long) div_up(nsite, 32 /
 
 int site_blocks(const mmnb_handle *h) { return site_grid(h->nsite, kMaxOrder); }
 
-// A lane per mesh plane up to this many sites, where a lane per site leaves most of the
-// chip idle.  The step in us, lanes per plane against per site: order 5 mixed, 650 sites
-// 28.0 and 29.9, 3,000 32.8 and 34.9, 8,700 42.1 and 43.5; with ik 1,500 32.4 and 37.5;
-// order 7 3,000 36.9 and 42.8; FP64 order 5 3,000 34.9 and 36.9, 8,700 53.8 and 55.4, order 7
-// 38.7 and 43.1, 62.5 and 64.4.  Past it (the weights repeated in each lane) order 5 mixed,
-// 16,500 sites 54.3 and 51.0, 33,000 75.4 and 68.5; FP64 80.1 and 76.3, 119.7 and 110.1.
-// Mixed orders up to 5 without ik, where the lanes gain least, take a lane per site from
-// 2,500 sites on: replicas that fill the chip together pay for the lanes' work (64 of 258
-// to 3,933 waters, 1,000 steps: 760 ms with 10,000 here, 731 with 2,500).
-constexpr int site_lanes_max(int P, MeshKind kind) { return kind == kMesh32 && P <= 5 ? 2500 : 10000; }
+// A lane per mesh plane up to this many sites, where a lane per site leaves much of the
+// chip idle.  Shuffled boxes, the step in us, lanes per plane against per site: with ik
+// 40,000, mixed order 4 12,288 sites 49.5 and 52.8, 36,000 82.9 and 86.8, order 7 68.8 and
+// 83.3, 139.8 and 155.6, FP64 order 5 76.2 and 84.2, 162.7 and 160.6, order 7 93 and 118,
+// 209 and 233; without, 14,000, FP64 order 5 10,500 sites 61.8 and 64.5, 15,000 80.1 and
+// 79.5, 36,000 129.7 and 125.1, mixed order 7 12,288 56.9 and 59.4, 36,000 102 and 98.
+// Mixed orders up to 5 without ik, where the lanes gain least (650 sites 28.0 and 29.9,
+// 3,000 32.8 and 34.9, 12,288 45.4 and 47.4, 24,000 63.1 and 62.2), take a lane per site
+// from 2,500 sites on: replicas that fill the chip together pay for the lanes' work (64 of
+// 258 to 3,933 waters, 1,000 steps: 760 ms with 10,000 here, 731 with 2,500).
+constexpr int site_lanes_max(int P, MeshKind kind)
+{
+  return kind == kMesh32Ik || kind == kMesh64Ik ? 40000 : kind == kMesh32 && P <= 5 ? 2500 : 14000;
+}
 // (site_words' loads, at 6 blocks an SM, want the chip filled: order 5 mixed, shuffled, point
 // by point against them: 18,000 sites 58.0 and 60.8, 36,000 74.7 and 75.1, 98,304 161 and 150)
 constexpr int kSiteWordsMin = 40000;
