@@ -83,7 +83,7 @@ typedef struct mmnb_config {
   double rspace_cutoff;          /* 0 -> 0.45 * minimum diameter */
   double smoothing_width;        /* 1 */
   double neighbor_list_width;    /* 0 -> 0.2 rc, clipped to 0.499 d - rc */
-  double kspace_cutoff;          /* 5 (ordinary Ewald |n| cutoff) */
+  double kspace_cutoff;          /* 5 (ordinary Ewald |n| cutoff; below 1008) */
   double ewald_screening;        /* -1 -> automatic: sqrt(pi kc / (rc d)) for the
                                     k-sum; with P3M the value that minimises the
                                     summed squares of the real-space and mesh error
